@@ -55,6 +55,23 @@ def test_quant_rows_bit_exact(cuda_dev, M, K, dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_quant_codes_at_rounding_ties(cuda_dev, dtype):
+    """One row per significand of the absmax, holding every value of the nine binades below it (for fp16 every fourth
+    significand and the exact half): the quotients that are rounding ties (absmax / 2 in every row, more where the
+    significand is a multiple of 127) and all their neighbours get the codes of the IEEE division."""
+    one, per = (0x3F80, 128) if dtype == torch.bfloat16 else (0x3C00, 1024)
+    amax = torch.arange(one, one + per, 1 if per == 128 else 4, dtype=torch.int32)
+    below = torch.arange(0, 9 * per, 1 if per == 128 else 4, dtype=torch.int32)
+    bits = torch.cat([amax[:, None], amax[:, None] - per, (amax[:, None] - below[None, :])], dim=1)
+    bits[:, 2::2] |= 0x8000                                          # alternate signs
+    bits = torch.nn.functional.pad(bits, (0, (-bits.shape[1]) % 16))
+    x = torch.where(bits >= 0x8000, bits - 0x10000, bits).to(torch.int16).view(dtype)
+    q, s = int8_exec.quant_rows(x.to(cuda_dev))
+    qo, so = oracle.quant_rows(x)
+    assert torch.equal(s.cpu(), so) and torch.equal(q.cpu(), qo)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_quant_scales_for_every_absmax(cuda_dev, dtype):
     """Every positive finite value of the activation type as a row's absmax: the scale equals the IEEE quotient
     absmax / 127 bit for bit (the kernel computes it with a multiply-and-correct sequence), and so do the group scales."""
