@@ -32,6 +32,8 @@ SIGNATURES = {
                                   c_void_p]),
     "pq_lowrank_down_cat": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int, c_void_p, c_int64, c_int,
                                     c_void_p, c_int64, c_int64, c_void_p, c_size_t, c_void_p]),
+    "pq_quant_rows_lowrank": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int, c_int64, c_void_p, c_int64,
+                                      c_int, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_size_t, c_void_p]),
     "pq_adaln_quant_rows": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int64, c_void_p, c_void_p, c_int64, c_int64,
                                     ctypes.c_float, c_void_p, c_int64, c_void_p, c_void_p, c_void_p]),
     "pq_gather_quant_rows": (c_int, [c_void_p, c_int, c_int64, c_int64, c_int64, c_void_p, c_int64, c_void_p,

@@ -11,6 +11,11 @@
 #include "gemm_common.cuh"
 
 namespace pq {
+// quant_down.cu: t alone, the columns summed in slices over a cluster
+bool lowrank_sliced(int64_t K, int R);
+int lowrank_down_sliced(const void* x0, int64_t K0, int64_t ldx0, const void* x1, int64_t K1, int64_t ldx1, int dtype,
+                        const void* a_t, int64_t lda, int R, void* t, int64_t ldt, int64_t M, void* workspace, size_t ws_bytes,
+                        void* stream);
 namespace {
 
 constexpr int LM = 64;                 // rows of x per tile (tcgen05 M = 64)
@@ -272,6 +277,9 @@ int lowrank_down_impl(const void* x, int64_t K0, int64_t ldx, const void* x1, in
   if (K1 > 0 && (K1 % 8 != 0 || ldx1 % 8 != 0 || !aligned_to(x1, 16))) return PQ_ERR_ALIGN;
   if (K1 > 0 && K0 % LKE != 0) return PQ_ERR_UNSUPPORTED;       // the seam has to fall between two 64-element boxes
   if (workspace != nullptr && ws_bytes < PQ_GEMM_WORKSPACE_BYTES) return PQ_ERR_WORKSPACE;
+  // one factor and rows of a certain length: the cluster kernel, whose t the fused quantisation + down-projection repeats
+  if (lowrank_sliced(K, R))
+    return lowrank_down_sliced(x, K0, ldx, x1, K1, ldx1, dtype, a_t, lda, R, t, ldt, M, workspace, ws_bytes, stream);
   const bool bf16 = dtype == PQ_DTYPE_BF16;
   CUtensorMap tmX, tmX1, tmA;
   int rc = make_map16(&tmX, x, M, K0, ldx, LM, bf16);

@@ -327,6 +327,19 @@ class Int8Linear(nn.Module):
             return ops.lowrank_down(x2, self._lr_At())
         return x2.to(self.lr_A.dtype) @ self.lr_A
 
+    def _one_launch_prologue(self, x2: torch.Tensor) -> bool:
+        return (self.lr_A.shape[1] == 32 and self.lr_A.dtype == x2.dtype and ops.quant_lowrank_ok(x2)
+                and not torch.compiler.is_compiling())
+
+    def _quant_down(self, x2: torch.Tensor):
+        """(codes, row scales, t) of the input of a layer with a low-rank branch: one launch where the library takes the
+        rows as they are, the two separate steps otherwise."""
+        if self._one_launch_prologue(x2):
+            return ops.quant_rows_lowrank(x2, self._lr_At())
+        t = self._down(x2)
+        xq, sx = quant_rows(x2)
+        return xq, sx, t
+
     def _fusable_lowrank(self, x2: torch.Tensor) -> bool:
         return (self.lr_A is not None and self.lr_A.shape[1] == 32 and x2.shape[1] % 32 == 0
                 and self.lr_A.dtype == x2.dtype and self.lr_B.dtype == x2.dtype and self.out_features % 8 == 0)
@@ -364,14 +377,18 @@ class Int8Linear(nn.Module):
         t_ptr = None
         ldt = 0
         if lr:
-            t = self._down(x2)                                  # [M, 32]
+            q, sx, t = self._quant_down(x2)                     # t [M, 32]
             t_ptr, ldt = t.data_ptr(), t.stride(0)
-        q = torch.empty((M, K), dtype=torch.int8, device=dev)
-        sx = torch.empty((M,), dtype=torch.float32, device=dev)
+        else:
+            q = torch.empty((M, K), dtype=torch.int8, device=dev)
+            sx = torch.empty((M,), dtype=torch.float32, device=dev)
         out = torch.empty((M, N), dtype=x2.dtype, device=dev)
         stream = ops._stream(x2)
         with ops._on_device(x2):
-            rc = lib.pq_quant_rows(x2.data_ptr(), code, M, K, x2.stride(0) if M > 1 else K, q.data_ptr(), sx.data_ptr(), stream)
+            rc = 0
+            if not lr:
+                rc = lib.pq_quant_rows(x2.data_ptr(), code, M, K, x2.stride(0) if M > 1 else K, q.data_ptr(), sx.data_ptr(),
+                                       stream)
             if rc == 0:
                 rc = lib.pq_int8_gemm(q.data_ptr(), K, sx.data_ptr(), wptr, ldw, sc_ptr, b_ptr, t_ptr, ldt, lb_ptr, ldb,
                                       lbt_ptr, 32 if lr else 0, code, out.data_ptr(), code, N, M, N, K, ws.data_ptr(),
@@ -427,8 +444,7 @@ class Int8Linear(nn.Module):
             xq, sx, T = grp.prepare(x2)
             t = grp.t_of(self, T) if lr else None
         else:
-            t = self._down(x2) if lr else None
-            xq, sx = quant_rows(x2)
+            xq, sx, t = self._prologue(x2)
         y2 = ops._gemm_impl(xq, sx, self.weight_int8, self.w_scale, self.bias, t, self.lr_B if lr else None, x2.dtype,
                             lb_t=self._lr_Bt() if lr else None, epilogue=epilogue,
                             out=out2 if (epilogue & ops.EPI_ACCUMULATE) else None)
@@ -471,15 +487,17 @@ class Int8Linear(nn.Module):
         if x_more is not None:
             if (ops.cat_sources_ok(x2, x_more) and not torch.compiler.is_compiling()
                     and (not lr or (self.lr_A.shape[1] == 32 and self.lr_A.dtype == x2.dtype))):
-                t = ops.lowrank_down_cat(x2, x_more, self._lr_At()) if lr else None
+                if lr:
+                    return ops.quant_rows_lowrank(x2, self._lr_At(), x_more)
                 xq, sx = ops.quant_rows_cat(x2, x_more)
-                return xq, sx, t
+                return xq, sx, None
             x2 = torch.cat([x2, x_more], dim=1)
         if x2.stride(1) != 1:
             x2 = x2.contiguous()
-        t = self._down(x2) if lr else None
+        if lr:
+            return self._quant_down(x2)
         xq, sx = quant_rows(x2)
-        return xq, sx, t
+        return xq, sx, None
 
     def forward_cat(self, x0: torch.Tensor, x1: torch.Tensor) -> torch.Tensor:
         """``self(torch.cat([x0, x1], dim=-1))`` without building the concatenated tensor: the single-stream blocks'
@@ -554,10 +572,7 @@ class Int8Linear(nn.Module):
             for o in out_more:
                 o.copy_(y, non_blocking=True)
             return out
-        if x2.stride(1) != 1:
-            x2 = x2.contiguous()
-        t = self._down(x2) if lr else None
-        xq, sx = quant_rows(x2)
+        xq, sx, t = self._prologue(x2)
         return ops._gemm_impl(xq, sx, self.weight_int8, self.w_scale, self.bias, t, self.lr_B if lr else None, x2.dtype,
                               lb_t=self._lr_Bt() if lr else None, out=out, out_more=list(out_more))
 
@@ -572,8 +587,7 @@ class Int8Linear(nn.Module):
         if x2.stride(1) != 1:
             x2 = x2.contiguous()
         if self._fusable_lowrank(x2):
-            t = self._down(x2)                                     # [M, r], rounded to the activation dtype
-            xq, sx = quant_rows(x2)
+            xq, sx, t = self._quant_down(x2)                       # t [M, r], rounded to the activation dtype
             y = int8_gemm_lr(xq, sx, self.weight_int8, self.w_scale, self.bias, t, self.lr_B, x2.dtype, self._lr_Bt())
             return y.reshape(*shape[:-1], self.out_features)
         y = int8_linear_2d(x2, self.weight_int8, self.w_scale, self.bias)
@@ -710,10 +724,11 @@ class Int8LinearRouted(Int8Linear):
             _LO_SCRATCH[key] = buf
         return ops.unpack_int4(p, buf.view(self.out_features, self.in_features))
 
-    def _two_tier(self, xq, sx, x_rows: Callable[[], torch.Tensor], m_hi: int, dtype: torch.dtype, fused: bool):
-        t = lb = lbt = None
+    def _two_tier(self, xq, sx, x_rows: Callable[[], torch.Tensor], m_hi: int, dtype: torch.dtype, fused: bool, t=None):
+        lb = lbt = None
         if fused:
-            t = self._down(x_rows())
+            if t is None:
+                t = self._down(x_rows())
             lb = self.lr_B; lbt = self._lr_Bt()
         y = int8_gemm_grouped(xq, sx, self.weight_int8, self.w_scale, self._lo_codes(), self.w_scale_lo,
                               self.bias, t, lb, m_hi, dtype, lbt)
@@ -724,8 +739,13 @@ class Int8LinearRouted(Int8Linear):
 
     def forward_rows(self, x2: torch.Tensor, m_hi: int) -> torch.Tensor:
         """x2 [M,K] already gathered and ordered hi-tier rows first."""
-        xq, sx = quant_rows(x2)
-        return self._two_tier(xq, sx, lambda: x2, m_hi, x2.dtype, self._fusable_lowrank(x2))
+        fused = self._fusable_lowrank(x2)
+        t = None
+        if fused:
+            xq, sx, t = self._quant_down(x2)
+        else:
+            xq, sx = quant_rows(x2)
+        return self._two_tier(xq, sx, lambda: x2, m_hi, x2.dtype, fused, t)
 
     def forward_gathered(self, canvas: torch.Tensor, row_idx: torch.Tensor, m_hi: int) -> torch.Tensor:
         """Gather + quantise in one kernel straight from the canvas, then the two-tier GEMM."""

@@ -283,6 +283,41 @@ def lowrank_down_ok(x2: Tensor) -> bool:
             and x2.shape[0] >= LOWRANK_DOWN_MIN_ROWS)
 
 
+# row lengths the one-launch form (pq_quant_rows_lowrank) is used for.  Below 512 columns a block is too little work for
+# its two sweeps and the exchange between them (65536 rows, one launch / two, us: 256 columns 23.0 / 19.5, 512 columns
+# 29.3 / 29.4, 1536 columns 71 / 85); above 16384 a column slice of A no longer fits beside the tiles.
+QUANT_LOWRANK_K = (512, 16384)
+
+
+def quant_lowrank_ok(x2: Tensor) -> bool:
+    """Inputs pq_quant_rows_lowrank takes without a copy and is the faster choice for."""
+    return lowrank_down_ok(x2) and QUANT_LOWRANK_K[0] <= x2.shape[1] <= QUANT_LOWRANK_K[1]
+
+
+def quant_rows_lowrank(x2: Tensor, a_t: Tensor, x_more: Optional[Tensor] = None) -> Tuple[Tensor, Tensor, Tensor]:
+    """(q, s, t): quant_rows and lowrank_down of x2 (or of [x2 | x_more]) in one launch that reads the rows once from memory
+    (pq_quant_rows_lowrank); a_t [32, K] contiguous."""
+    M, K0 = x2.shape
+    K1 = x_more.shape[1] if x_more is not None else 0
+    K = K0 + K1
+    assert x2.stride(1) == 1 and (x_more is None or cat_sources_ok(x2, x_more))
+    assert a_t.dtype == x2.dtype and a_t.shape == (32, K) and a_t.is_contiguous() and a_t.device == x2.device
+    dev = x2.device
+    q = torch.empty((M, K), dtype=torch.int8, device=dev)
+    s = torch.empty((M,), dtype=torch.float32, device=dev)
+    t = torch.empty((M, 32), dtype=x2.dtype, device=dev)
+    ws = status_word(dev)
+    ld0 = x2.stride(0) if M > 1 else max(K0, x2.stride(0))
+    ld1 = 0 if x_more is None else (x_more.stride(0) if M > 1 else max(K1, x_more.stride(0)))
+    with _on_device(x2):
+        rc = _LIB().pq_quant_rows_lowrank(x2.data_ptr(), K0, ld0, _ptr(x_more), K1, ld1, _dt(x2.dtype), M, a_t.data_ptr(), K, 32,
+                                          q.data_ptr(), s.data_ptr(), t.data_ptr(), 32, ws.data_ptr(), ws.numel() * 4,
+                                          _stream(x2))
+    if rc:
+        _lib.check(rc, f"pq_quant_rows_lowrank(M={M}, K={K0}+{K1})")
+    return q, s, t
+
+
 # ------------------------------------------------------------------------------------------------ 4-bit storage
 def pack_int4(codes: Tensor) -> Tensor:
     """int8 codes in [-8, 7], shape [N, K] with K even -> uint8 [N, K/2]: element 2b in the low nibble of byte b,

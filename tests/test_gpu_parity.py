@@ -1138,3 +1138,39 @@ def test_bounded_wait_runs_out_and_is_reported(cuda_dev):
     ops.check_device_status(cuda_dev)                               # the word was cleared by the read above
     run_gemm_case(cuda_dev, 300, 512, 256, lowrank=True, bias=True, seed=5)
     run_gemm_case(cuda_dev, 2049, 768, 384, lowrank=False, bias=True, seed=6)
+
+
+# ------------------------------------------------------------------------------------------------ quantisation + down-projection
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,K1", [(1, 64, 0), (63, 128, 0), (64, 200, 0), (65, 1288, 0), (200, 1536, 0), (130, 1544, 0),
+                                    (1000, 3072, 0), (9473, 3072, 0), (700, 6152, 0), (513, 12288, 0), (1300, 15360, 0),
+                                    (96, 16384, 0), (2600, 192, 0), (130, 64, 8), (700, 3072, 12288), (5000, 1024, 520)])
+def test_quant_rows_lowrank(cuda_dev, M, K, K1, dtype):
+    """Codes and scales equal the quantiser's bit for bit; t lies within one unit in the last place of the fp64 product (plus
+    the bound of an fp32 summation in any order).  Row and K tails, strided rows, slices of the last CTA that are short or
+    empty, one to eight CTAs per row block, several blocks per CTA, two sources."""
+    g = torch.Generator().manual_seed(M + K + K1)
+    Kt = K + K1
+    xp = torch.randn(M, Kt + 16, generator=g)
+    xp[:, torch.randperm(Kt, generator=g)[: max(1, Kt // 200)]] *= 20.0
+    xp = xp.to(dtype)
+    x = xp[:, :Kt].contiguous()
+    if M > 3:
+        xp[2].zero_(); x[2].zero_()
+    A = (torch.randn(Kt, 32, generator=g) * 0.05).to(dtype)
+    a_t = A.t().contiguous().to(cuda_dev)
+    xd = xp.to(cuda_dev)
+    x0, x1 = xd[:, :K], xd[:, K:Kt] if K1 else None
+    if K1 and x1.data_ptr() % 16:
+        x1 = x1.contiguous()
+    q, s, t = ops.quant_rows_lowrank(x0, a_t, x1)
+    qs, ss = int8_exec.quant_rows(x.to(cuda_dev))
+    assert torch.equal(q, qs) and torch.equal(s, ss)
+    ref = x.to(cuda_dev).double() @ A.to(cuda_dev).double()
+    mag = x.to(cuda_dev).double().abs() @ A.to(cuda_dev).double().abs()
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    err = (t.double() - ref).abs()
+    assert bool((err <= ulp * ref.abs() * 1.01 + 1e-6 * mag).all()), err.max().item()
+    if Kt >= 512 and not K1:
+        assert torch.equal(t, ops.lowrank_down(x0, a_t))              # the same slices, summed in the same order
+        assert torch.equal(t[: M // 2], ops.quant_rows_lowrank(x0[: M // 2], a_t)[2])   # whatever the number of rows
