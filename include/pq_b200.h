@@ -65,8 +65,7 @@ int pq_last_cuda_error(void);
  *                       schedule (the rows of a panel stay in L2 across the rounds); 0 = one panel over all rows;
  *   "gemm_l2_hints"     CTA-pair kernel, L2 eviction priorities: bit 0 weights evict-last, bit 1 activations evict-first,
  *                       bit 2 activations evict-last, bit 3 streaming output stores;
- *   "g32_variant"       group-32 GEMM: bit 0 = eight epilogue warps instead of sixteen; bit 1 = scalar instead of packed
- *                       fp32 operations; bit 3 = data path only (measurements; the output is meaningless).
+ *   "g32_variant"       group-32 GEMM: 0 = tile width by the size of the launch, 1 = 128 columns, 2 = 64 columns.
  * Unknown keys return PQ_ERR_UNSUPPORTED.  Not part of the reference API. */
 int pq_set_option(const char* key, int value);
 int pq_get_option(const char* key, int* value);

@@ -48,7 +48,7 @@ struct Options {
   int gemm_tail_pairs = 1; // CTA-pair kernel: SM pairs that the pm x pn grid leaves over take a tail region of the tiles (0: they idle)
   int gemm_panel_mb = 0;   // CTA-pair kernel, several column rounds: megabytes of activation rows per row panel (0 = one panel)
   int gemm_l2_hints = 0;   // CTA-pair kernel: bit 0 weights evict-last, bit 1 activations evict-first, bit 2 activations evict-last, bit 3 streaming output stores
-  int g32_variant = 0;     // group-32 GEMM: bit 0 eight epilogue warps, bit 1 scalar fp32 operations, bit 3 data path only
+  int g32_variant = 0;     // group-32 GEMM tiles: 0 by the size of the launch, 1 128 columns, 2 64 columns
 };
 Options& options();
 

@@ -25,13 +25,19 @@
 // 160-200 bytes per cycle, not a latency one.  Drain (about 320) and arithmetic (about 310: the conversion pipe takes
 // 256 of them) add up instead of overlapping, whatever the warps' arrangement: requesting the next chunk only after
 // the current one has been folded, i.e. with no overlap by construction, measures the same (415 against 406 TOPS).
-// Tried and dropped: slots handed over one by one with the next chunk always requested across slot and stage boundaries
-// (non-blocking probe of the next slot's barrier): 356 instead of 408 TOPS, spills at 96 registers;
-// a row-per-thread arrangement (tcgen05.ld 32x32b: the row scale becomes a register, but the loads
-// are no faster and the column scales need twice the shared-memory loads); accumulators pre-biased with 0x4B400000 so
-// that the int32 result read as fp32 bits needs only a subtraction (the tcgen05.st that restores the bias costs more
-// tensor-memory bandwidth than the integer additions it saves); keeping a load in flight across slot pairs, stages and
-// tiles (more live registers than the 96 per thread that 18 warps leave).
+// Tried and dropped, 16384 x 1280 -> 10240 (1050 us as it stands): slots handed over one by one with the next chunk always
+// requested across slot and stage boundaries: 356 instead of 408 TOPS, spills at 96 registers; the row-per-thread load form
+// (tcgen05.ld 32x32b moves the 64 KB of a tile and group in 72 cycles where this one, which fills sixteen lanes at a time,
+// takes 256, but its column scales need twice the shared-memory bytes, and one slot at a time the chain of load, fold and
+// hand-over is 1330 us long); codes held as fp16, whose kind::f16 partial sums arrive as floats (995 us, for two more bytes
+// per weight at rest); mma.sync, which leaves the partial sums in the registers of the folding warp (470 cycles per tile and
+// group in a register loop, 1330 us once the fragments come through shared memory); accumulators pre-biased with
+// 0x4B400000 so that the int32 result read as fp32 bits needs only a subtraction (the tcgen05.st that restores the bias
+// costs more tensor-memory bandwidth than the integer additions it saves); keeping a load in flight across slot pairs,
+// stages and tiles (more live registers than the 96 per thread that 18 warps leave).
+// Tile width: 128 columns, 64 where 128-column tiles would leave half of the SMs or more without one (a tile's chain of
+// hand-overs is then shorter and twice as many SMs work: 1024 x 2560 -> 640 33.2 -> 23.5 us, 77 x 640 -> 5120 12.6 -> 10.5 us);
+// with enough tiles the wide form is ahead (4096 x 1280 -> 1280 51.7 against 55.8 us).
 // Roles: warp 0 TMA producer (operand stages plus a ring of scale tiles), warp 1 MMA issuer, warps 2.. epilogue.
 // Every wait is bounded.  No clusters, no multicast.
 #include <type_traits>
@@ -41,15 +47,20 @@
 namespace pq {
 namespace {
 
-constexpr int GBN = 128;                 // columns per tile = one tensor-memory slot
-constexpr int kSlots = 4;
-constexpr int kSlotPairs = 2;
-constexpr int kG32Stages = 4;
 constexpr int kGroupsPerStage = BK / 32;  // 4
-constexpr int g32_threads(int ew) { return 64 + 32 * ew; }
+constexpr int kG32EpiWarps = 16;
+constexpr int kG32Threads = 64 + 32 * kG32EpiWarps;
 
-__device__ __forceinline__ void tmem_ld_cols(uint32_t addr, uint32_t (&v)[32]) { tmem_ld_16x256b_x8(addr, v); }
+// 16 lanes x 16 columns, the arrangement of tmem_ld_16x256b_x4
+__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+      : "r"(taddr)
+      : "memory");
+}
 __device__ __forceinline__ void tmem_ld_cols(uint32_t addr, uint32_t (&v)[16]) { tmem_ld_16x256b_x4(addr, v); }
+__device__ __forceinline__ void tmem_ld_cols(uint32_t addr, uint32_t (&v)[8]) { tmem_ld_16x256b_x2(addr, v); }
 
 struct G32Params {
   const float* bias;
@@ -61,38 +72,42 @@ struct G32Params {
   int has_bias;
 };
 
+template <int BN>
 struct G32Smem {
+  static constexpr int kStages = 4;
   static constexpr int kABytes = BM * BK;
-  static constexpr int kBBytes = GBN * BK;
+  static constexpr int kBBytes = BN * BK;
   static constexpr int kStageBytes = kABytes + kBBytes;
   static constexpr int kSaBytes = BM * kGroupsPerStage * 4;     // [128 rows][4 groups] fp32
-  static constexpr int kSwBytes = kGroupsPerStage * GBN * 4;    // [4 groups][128 cols] fp32
+  static constexpr int kSwBytes = kGroupsPerStage * BN * 4;     // [4 groups][BN cols] fp32
   static constexpr int kScaleBytes = kSaBytes + kSwBytes;
-  static constexpr int kScaleOff = kG32Stages * kStageBytes;
-  static constexpr int kBarOff = kScaleOff + kG32Stages * kScaleBytes;
-  static constexpr int kNumBars = 4 * kG32Stages + 2 * kSlotPairs;
+  static constexpr int kScaleOff = kStages * kStageBytes;
+  static constexpr int kSlotPairs = 256 / BN;                   // two slots of BN tensor-memory columns each
+  static constexpr int kBarOff = kScaleOff + kStages * kScaleBytes;
+  static constexpr int kNumBars = 4 * kStages + 2 * kSlotPairs;
   static constexpr int kMiscOff = kBarOff + kNumBars * 8;
   static constexpr int kDynamic = kMiscOff + 16 + 1024;
 };
 
-// EW epilogue warps; ARITH = false replaces the scale arithmetic by a plain sum (measurement of the data path only, the
-// output is then meaningless); PACKED = false uses scalar instead of packed fp32 operations.
-template <typename OutT, int EW, bool ARITH, bool PACKED>
-__global__ void __launch_bounds__(g32_threads(EW), 1)
+template <typename OutT, int BN>
+__global__ void __launch_bounds__(kG32Threads, 1)
 pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
                         const __grid_constant__ CUtensorMap tmSa, const __grid_constant__ CUtensorMap tmSw,
                         const G32Params p) {
-  using L = G32Smem;
-  static_assert(EW == 8 || EW == 16, "eight or sixteen epilogue warps");
-  constexpr int kColW = GBN / (EW / 4);       // columns of the tile per epilogue warp: 64 or 32
-  constexpr int kNB = kColW / 8;              // 8-column blocks per warp: 8 or 4
+  using L = G32Smem<BN>;
+  constexpr int kStages = L::kStages, kSlotPairs = L::kSlotPairs;
+  constexpr int kColW = BN / 4;               // columns of the tile per epilogue warp: 32 or 16
+  constexpr int kNB = kColW / 8;              // 8-column blocks per warp
+  // stage n fills (and drains) slot pairs 0 and 1, or with four pairs 0, 1 and 2, 3 in turn
+  auto slot_pair = [](uint32_t n, int h) -> uint32_t { return kSlotPairs == 2 ? h : ((n & 1u) << 1) + h; };
+  auto pair_parity = [](uint32_t n) -> uint32_t { return (kSlotPairs == 2 ? n : n >> 1) & 1u; };
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
-  uint64_t* empty_bar = full_bar + kG32Stages;
-  uint64_t* sfull_bar = empty_bar + kG32Stages;
-  uint64_t* sempty_bar = sfull_bar + kG32Stages;
-  uint64_t* slot_full = sempty_bar + kG32Stages;      // [pair]
+  uint64_t* empty_bar = full_bar + kStages;
+  uint64_t* sfull_bar = empty_bar + kStages;
+  uint64_t* sempty_bar = sfull_bar + kStages;
+  uint64_t* slot_full = sempty_bar + kStages;      // [pair]
   uint64_t* slot_empty = slot_full + kSlotPairs;      // [pair]
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(smem + L::kMiscOff);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L::kMiscOff + 4);
@@ -100,17 +115,17 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int mt_total = (p.M + BM - 1) / BM;
-  const int nt = (p.N + GBN - 1) / GBN;
+  const int nt = (p.N + BN - 1) / BN;
   const int num_kb = p.K / BK;                      // host guarantees K % 128 == 0
-  constexpr uint32_t kTmemCols = kSlots * GBN;      // 512
+  constexpr uint32_t kTmemCols = 512;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmSa); tma_prefetch_desc(&tmSw);
-    for (int s = 0; s < kG32Stages; ++s) {
+    for (int s = 0; s < kStages; ++s) {
       mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1);
-      mbar_init(&sfull_bar[s], 1); mbar_init(&sempty_bar[s], EW);
+      mbar_init(&sfull_bar[s], 1); mbar_init(&sempty_bar[s], kG32EpiWarps);
     }
-    for (int s = 0; s < kSlotPairs; ++s) { mbar_init(&slot_full[s], 1); mbar_init(&slot_empty[s], EW); }
+    for (int s = 0; s < kSlotPairs; ++s) { mbar_init(&slot_full[s], 1); mbar_init(&slot_empty[s], kG32EpiWarps); }
     *abort_flag = 0;
     fence_mbar_init();
     fence_proxy_async_smem();
@@ -128,7 +143,7 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
       TileWalker w; w.init(p.sched_pm, p.sched_pn, mt_total, nt);
 #pragma unroll 1
       for (; w.valid() && ok; w.advance()) {
-        const int row0 = w.mt * BM, n0 = w.ntile * GBN;
+        const int row0 = w.mt * BM, n0 = w.ntile * BN;
 #pragma unroll 1
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!wait_or_abort(&empty_bar[stage], phase ^ 1u, abort_flag) ||
@@ -144,12 +159,12 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
           tma_load_2d(sc_s, &tmSa, &sfull_bar[stage], kb * kGroupsPerStage, row0);           // [128 rows][4 groups]
           tma_load_2d(sc_s + L::kSaBytes, &tmSw, &sfull_bar[stage], n0, kb * kGroupsPerStage);  // [4 groups][128 cols]
           ++issued;
-          if (++stage == kG32Stages) { stage = 0; phase ^= 1u; }
+          if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
       }
-      const int pending = issued < kG32Stages ? static_cast<int>(issued) : kG32Stages;
+      const int pending = issued < kStages ? static_cast<int>(issued) : kStages;
       for (int i = 0; i < pending; ++i) {          // copies in flight must land before the CTA may exit
-        if (--stage < 0) { stage = kG32Stages - 1; phase ^= 1u; }
+        if (--stage < 0) { stage = kStages - 1; phase ^= 1u; }
         if (!wait_or_abort(&full_bar[stage], phase, abort_flag) || !wait_or_abort(&sfull_bar[stage], phase, abort_flag)) {
           for (int k = 0; k < 64; ++k) __nanosleep(1000);
           break;
@@ -157,11 +172,11 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
       }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer: one instruction per group
+    // ------------------------------------------------------------------ MMA issuer: a fresh accumulator per group
     if (elect_one()) {
-      constexpr uint32_t idesc = make_idesc_i8(BM, GBN);
+      constexpr uint32_t idesc = make_idesc_i8(BM, BN);
       int stage = 0; uint32_t phase = 0; bool ok = true;
-      uint32_t uses = 0;                              // stages issued so far = uses of either slot pair
+      uint32_t uses = 0;                              // stages issued so far: a stage fills two slot pairs
       TileWalker w; w.init(p.sched_pm, p.sched_pn, mt_total, nt);
 #pragma unroll 1
       for (; w.valid() && ok; w.advance()) {
@@ -175,16 +190,16 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
           const uint64_t a_desc = make_kmajor_sw128_desc(a_addr);
           const uint64_t b_desc = make_kmajor_sw128_desc(a_addr + L::kABytes);
 #pragma unroll
-          for (int pr = 0; pr < kSlotPairs; ++pr) {
-            // the epilogue's initial hand-over is completion 0 of slot_empty: use n of a pair waits for completion n
-            if (!wait_or_abort(&slot_empty[pr], uses & 1u, abort_flag)) {
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t pr = slot_pair(uses, h);
+            if (!wait_or_abort(&slot_empty[pr], pair_parity(uses) ^ 1u, abort_flag)) {
               report_timeout(p.status, 2, 2); *abort_flag = 1; ok = false; break;
             }
             tc_fence_after();
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-              const int g = 2 * pr + j;
-              tc_mma_i8(tmem_base + g * GBN, a_desc + static_cast<uint64_t>(2 * g), b_desc + static_cast<uint64_t>(2 * g),
+              const int g = 2 * h + j;
+              tc_mma_i8(tmem_base + (2 * pr + j) * BN, a_desc + static_cast<uint64_t>(2 * g), b_desc + static_cast<uint64_t>(2 * g),
                         idesc, 0u);
             }
             tc_commit(&slot_full[pr]);
@@ -192,7 +207,7 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
           if (!ok) break;
           ++uses;
           tc_commit(&empty_bar[stage]);
-          if (++stage == kG32Stages) { stage = 0; phase ^= 1u; }
+          if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
       }
     }
@@ -209,18 +224,17 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
     const bool vec_store = (p.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
     bool aborted = false;
     int stage = 0; uint32_t phase = 0;
-    uint32_t uses = 0;
-    // lanes [32 quarter + 16 h, +16), this warp's columns, of slot g
-    auto slot_addr = [&](int g, int h) {
-      return tmem_base + static_cast<uint32_t>(g * GBN + colg * kColW) + (static_cast<uint32_t>(quarter * 32 + h * 16) << 16);
+    uint32_t uses = 0;                         // stages consumed so far
+    // lanes [32 quarter + 16 h, +16), this warp's columns, of slot j of a pair
+    const uint32_t t_warp = tmem_base + static_cast<uint32_t>(colg * kColW) + (static_cast<uint32_t>(quarter * 32) << 16);
+    auto slot_addr = [&](uint32_t pr, int j, int h) {
+      return t_warp + (2 * pr + j) * BN + (static_cast<uint32_t>(h * 16) << 16);
     };
-    // the slots start out free
-    if (lane == 0) { mbar_arrive(&slot_empty[0]); mbar_arrive(&slot_empty[1]); }
 
     TileWalker w; w.init(p.sched_pm, p.sched_pn, mt_total, nt);
 #pragma unroll 1
     for (; w.valid() && !aborted; w.advance()) {
-      const int row0 = w.mt * BM, n0 = w.ntile * GBN;
+      const int row0 = w.mt * BM, n0 = w.ntile * BN;
       // y[h][nb][0] = (row 16 h + g4, cols 2q, 2q+1 of 8-column block nb), y[h][nb][1] = same columns, row + 8
       float2 y[2][kNB][2];
 #pragma unroll
@@ -241,14 +255,15 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         uint32_t va[4 * kNB], vb[4 * kNB];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const int g = k >> 1, h = k & 1, pr = k >> 2;
+          const int g = k >> 1, h = k & 1;
+          const uint32_t pr = slot_pair(uses, k >> 2);
           uint32_t (&v)[4 * kNB] = h == 0 ? va : vb;
           uint32_t (&vnext)[4 * kNB] = h == 0 ? vb : va;
           if ((k & 3) == 0) {                                        // first chunk of a pair: the MMAs have completed
-            const bool landed = wait_or_abort(&slot_full[pr], uses & 1u, abort_flag);
+            const bool landed = wait_or_abort(&slot_full[pr], pair_parity(uses), abort_flag);
             if (!__all_sync(0xffffffffu, landed)) { report_timeout(p.status, 3, 3); *abort_flag = 1; aborted = true; break; }
             tc_fence_after();
-            tmem_ld_cols(slot_addr(g, 0), v);
+            tmem_ld_cols(slot_addr(pr, 0, 0), v);
           }
           tc_wait_ld();                                              // chunk k is in v
           if ((k & 3) == 3) {                                        // the pair is in registers: hand it back
@@ -256,29 +271,19 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             __syncwarp();
             if (lane == 0) mbar_arrive(&slot_empty[pr]);
           } else {
-            tmem_ld_cols(slot_addr((k + 1) >> 1, (k + 1) & 1), vnext);   // on its way while chunk k is folded
+            tmem_ld_cols(slot_addr(pr, ((k + 1) >> 1) & 1, (k + 1) & 1), vnext);   // on its way while chunk k is folded
           }
           const float sa_lo = sa_row[(16 * h) * kGroupsPerStage + g], sa_hi = sa_row[(16 * h + 8) * kGroupsPerStage + g];
-          const float* swp = sw_s + g * GBN + colg * kColW + 2 * q;
+          const float* swp = sw_s + g * BN + colg * kColW + 2 * q;
 #pragma unroll
           for (int nb = 0; nb < kNB; ++nb) {
             // column scales: one 8-byte load per 8-column block serves the thread's two rows of this chunk
             const float2 sw2 = *reinterpret_cast<const float2*>(swp + nb * 8);
             const float2 pA = make_float2(__int2float_rn(static_cast<int32_t>(v[4 * nb + 0])), __int2float_rn(static_cast<int32_t>(v[4 * nb + 1])));
             const float2 pB = make_float2(__int2float_rn(static_cast<int32_t>(v[4 * nb + 2])), __int2float_rn(static_cast<int32_t>(v[4 * nb + 3])));
-            if constexpr (!ARITH) {
-              y[h][nb][0] = __fadd2_rn(make_float2(__uint_as_float(v[4 * nb + 0]), __uint_as_float(v[4 * nb + 1])), y[h][nb][0]);
-              y[h][nb][1] = __fadd2_rn(make_float2(__uint_as_float(v[4 * nb + 2]), __uint_as_float(v[4 * nb + 3])), y[h][nb][1]);
-            } else if constexpr (PACKED) {
-              // same arithmetic as the CPU restatement: running sum = fma(partial, s_a * s_w, running sum)
-              y[h][nb][0] = __ffma2_rn(pA, __fmul2_rn(make_float2(sa_lo, sa_lo), sw2), y[h][nb][0]);
-              y[h][nb][1] = __ffma2_rn(pB, __fmul2_rn(make_float2(sa_hi, sa_hi), sw2), y[h][nb][1]);
-            } else {
-              y[h][nb][0].x = __fmaf_rn(pA.x, __fmul_rn(sa_lo, sw2.x), y[h][nb][0].x);
-              y[h][nb][0].y = __fmaf_rn(pA.y, __fmul_rn(sa_lo, sw2.y), y[h][nb][0].y);
-              y[h][nb][1].x = __fmaf_rn(pB.x, __fmul_rn(sa_hi, sw2.x), y[h][nb][1].x);
-              y[h][nb][1].y = __fmaf_rn(pB.y, __fmul_rn(sa_hi, sw2.y), y[h][nb][1].y);
-            }
+            // same arithmetic as the CPU restatement: running sum = fma(partial, s_a * s_w, running sum)
+            y[h][nb][0] = __ffma2_rn(pA, __fmul2_rn(make_float2(sa_lo, sa_lo), sw2), y[h][nb][0]);
+            y[h][nb][1] = __ffma2_rn(pB, __fmul2_rn(make_float2(sa_hi, sa_hi), sw2), y[h][nb][1]);
           }
         }
         if (aborted) break;
@@ -286,7 +291,7 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         // scales of this stage consumed
         __syncwarp();
         if (lane == 0) mbar_arrive(&sempty_bar[stage]);
-        if (++stage == kG32Stages) { stage = 0; phase ^= 1u; }
+        if (++stage == kStages) { stage = 0; phase ^= 1u; }
       }
       if (aborted) break;
 
@@ -296,11 +301,12 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
         const int rA = row0 + quarter * 32 + h * 16 + g4;
         const int rB = rA + 8;
 #pragma unroll
-        for (int grp = 0; grp < kColW / 32; ++grp) {
+        for (int grp = 0; grp < (kColW + 31) / 32; ++grp) {
           uint32_t wA[4], wB[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int nb = grp * 4 + j;
+            if (nb >= kNB) { wA[j] = wB[j] = 0u; continue; }
             const int col = n0 + colg * kColW + nb * 8 + 2 * q;
             float2 b2 = make_float2(0.f, 0.f);
             if (p.has_bias && col + 1 < p.N) b2 = *reinterpret_cast<const float2*>(p.bias + col);
@@ -310,13 +316,15 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
             wB[j] = pack2(b.x, b.y, OutT{});
           }
           const int col_grp = n0 + colg * kColW + grp * 32;
-          if (vec_store && col_grp + 32 <= p.N) {
+          if (vec_store && col_grp + (kColW < 32 ? kColW : 32) <= p.N) {
             quad_transpose(wA, q);
             quad_transpose(wB, q);
-            if (rA < p.M) st_v4(out + static_cast<int64_t>(rA) * p.ldo + col_grp + q * 8, make_uint4(wA[0], wA[1], wA[2], wA[3]));
-            if (rB < p.M) st_v4(out + static_cast<int64_t>(rB) * p.ldo + col_grp + q * 8, make_uint4(wB[0], wB[1], wB[2], wB[3]));
+            const bool mine = q * 8 < kColW;             // sixteen columns: two lanes of a quad have a piece of the row
+            if (mine && rA < p.M) st_v4(out + static_cast<int64_t>(rA) * p.ldo + col_grp + q * 8, make_uint4(wA[0], wA[1], wA[2], wA[3]));
+            if (mine && rB < p.M) st_v4(out + static_cast<int64_t>(rB) * p.ldo + col_grp + q * 8, make_uint4(wB[0], wB[1], wB[2], wB[3]));
           } else {
-            store_pairs_slow(p.out, p.ldo, rA, rB, col_grp + 2 * q, p.M, p.N, make_uint4(wA[0], wA[1], wA[2], wA[3]),
+            const int lim = n0 + (colg + 1) * kColW < p.N ? n0 + (colg + 1) * kColW : p.N;
+            store_pairs_slow(p.out, p.ldo, rA, rB, col_grp + 2 * q, p.M, lim, make_uint4(wA[0], wA[1], wA[2], wA[3]),
                              make_uint4(wB[0], wB[1], wB[2], wB[3]));
           }
         }
@@ -336,31 +344,28 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
   }
 }
 
-template <typename OutT, int EW, bool ARITH, bool PACKED>
-int launch_g32_variant(const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtensorMap& tmSa, const CUtensorMap& tmSw,
-                       const G32Params& p, int grid, cudaStream_t st) {
-  auto kern = pq_int8_gemm_g32_kernel<OutT, EW, ARITH, PACKED>;
-  PQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, G32Smem::kDynamic));
-  kern<<<grid, g32_threads(EW), G32Smem::kDynamic, st>>>(tmA, tmW, tmSa, tmSw, p);
+template <typename OutT, int BN>
+int launch_g32(const int8_t* xq, int64_t ldx, const float* s_a, const int8_t* w, int64_t ldw, const float* s_w, G32Params p,
+               cudaStream_t st) {
+  using L = G32Smem<BN>;
+  const int64_t G = p.K / 32;
+  CUtensorMap tmA, tmW, tmSa, tmSw;
+  int rc = make_tile_map(&tmA, xq, p.M, p.K, ldx, BM);
+  if (rc != PQ_OK) return rc;
+  rc = make_tile_map(&tmW, w, p.N, p.K, ldw, BN);
+  if (rc != PQ_OK) return rc;
+  rc = make_f32_map(&tmSa, s_a, p.M, G, G, kGroupsPerStage, BM);      // [M, G]: box 4 groups x 128 rows
+  if (rc != PQ_OK) return rc;
+  rc = make_f32_map(&tmSw, s_w, G, p.N, p.N, BN, kGroupsPerStage);    // [G, N]: box BN cols x 4 groups
+  if (rc != PQ_OK) return rc;
+  const int mt = (p.M + BM - 1) / BM, ntl = (p.N + BN - 1) / BN;
+  const int max_ctas = options().gemm_max_ctas > 0 ? options().gemm_max_ctas : sm_count();
+  choose_cta_grid(mt, ntl, max_ctas, &p.sched_pm, &p.sched_pn);
+  auto kern = pq_int8_gemm_g32_kernel<OutT, BN>;
+  PQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kDynamic));
+  kern<<<p.sched_pm * p.sched_pn, kG32Threads, L::kDynamic, st>>>(tmA, tmW, tmSa, tmSw, p);
   PQ_CUDA_TRY(cudaGetLastError());
   return PQ_OK;
-}
-
-// Option "g32_variant": bit 0 = eight epilogue warps (default sixteen); bit 1 = scalar instead of packed fp32
-// operations; bit 3 = data path only (no scale arithmetic: for measurements, output meaningless).
-template <typename OutT, int EW>
-int launch_g32_e(int v, const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtensorMap& tmSa, const CUtensorMap& tmSw,
-                 const G32Params& p, int grid, cudaStream_t st) {
-  if (v & 8) return launch_g32_variant<OutT, EW, false, true>(tmA, tmW, tmSa, tmSw, p, grid, st);
-  if (v & 2) return launch_g32_variant<OutT, EW, true, false>(tmA, tmW, tmSa, tmSw, p, grid, st);
-  return launch_g32_variant<OutT, EW, true, true>(tmA, tmW, tmSa, tmSw, p, grid, st);
-}
-template <typename OutT>
-int launch_g32(const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtensorMap& tmSa, const CUtensorMap& tmSw,
-               const G32Params& p, int grid, cudaStream_t st) {
-  const int v = options().g32_variant;
-  if (v & 1) return launch_g32_e<OutT, 8>(v, tmA, tmW, tmSa, tmSw, p, grid, st);
-  return launch_g32_e<OutT, 16>(v, tmA, tmW, tmSa, tmSw, p, grid, st);
 }
 
 }  // namespace
@@ -377,33 +382,29 @@ extern "C" int pq_int8_gemm_g32(const int8_t* xq, int64_t ldx, const float* s_a,
   if (M == 0) return PQ_OK;
   if (xq == nullptr || s_a == nullptr || w == nullptr || s_w == nullptr || out == nullptr) return PQ_ERR_NULL;
   if (ldx < K || ldw < K || ldo < N) return PQ_ERR_SHAPE;
-  if (K % BK != 0) return PQ_ERR_UNSUPPORTED;            // whole 128-byte stages only (four groups per stage)
+  if (K % BK != 0) return PQ_ERR_UNSUPPORTED;            // whole stages only (four groups per stage)
   if (ldx % 16 != 0 || ldw % 16 != 0 || N % 4 != 0) return PQ_ERR_ALIGN;
   if (!aligned_to(xq, 16) || !aligned_to(w, 16) || !aligned_to(s_a, 16) || !aligned_to(s_w, 16)) return PQ_ERR_ALIGN;
   if (ldo % 2 != 0 || !aligned_to(out, 4)) return PQ_ERR_ALIGN;
   if (bias != nullptr && !aligned_to(bias, 8)) return PQ_ERR_ALIGN;
   if (workspace != nullptr && ws_bytes < PQ_GEMM_WORKSPACE_BYTES) return PQ_ERR_WORKSPACE;
 
-  const int64_t G = K / 32;
-  CUtensorMap tmA, tmW, tmSa, tmSw;
-  int rc = make_tile_map(&tmA, xq, M, K, ldx, BM);
-  if (rc != PQ_OK) return rc;
-  rc = make_tile_map(&tmW, w, N, K, ldw, GBN);
-  if (rc != PQ_OK) return rc;
-  rc = make_f32_map(&tmSa, s_a, M, G, G, kGroupsPerStage, BM);      // [M, G]: box 4 groups x 128 rows
-  if (rc != PQ_OK) return rc;
-  rc = make_f32_map(&tmSw, s_w, G, N, N, GBN, kGroupsPerStage);     // [G, N]: box 128 cols x 4 groups
-  if (rc != PQ_OK) return rc;
-
   G32Params p;
   p.bias = bias; p.out = out; p.status = static_cast<int32_t*>(workspace); p.ldo = ldo;
   p.M = static_cast<int>(M); p.N = static_cast<int>(N); p.K = static_cast<int>(K);
   p.has_bias = bias != nullptr ? 1 : 0;
-  const int mt = static_cast<int>((M + BM - 1) / BM), ntl = static_cast<int>((N + GBN - 1) / GBN);
-  const int max_ctas = options().gemm_max_ctas > 0 ? options().gemm_max_ctas : sm_count();
-  choose_cta_grid(mt, ntl, max_ctas, &p.sched_pm, &p.sched_pn);
-  const int grid = p.sched_pm * p.sched_pn;
+  p.sched_pm = p.sched_pn = 1;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (out_dtype == PQ_DTYPE_BF16) return launch_g32<__nv_bfloat16>(tmA, tmW, tmSa, tmSw, p, grid, st);
-  return launch_g32<__half>(tmA, tmW, tmSa, tmSw, p, grid, st);
+  // 64-column tiles where 128-column ones would leave half of the SMs or more without a tile
+  const int64_t tiles128 = ((M + BM - 1) / BM) * ((N + 127) / 128);
+  const int v = options().g32_variant;
+  const bool narrow = v == 2 || (v != 1 && 2 * tiles128 <= sm_count());
+  const bool bf16 = out_dtype == PQ_DTYPE_BF16;
+  if (narrow) {
+    if (bf16) return launch_g32<__nv_bfloat16, 64>(xq, ldx, s_a, w, ldw, s_w, p, st);
+    return launch_g32<__half, 64>(xq, ldx, s_a, w, ldw, s_w, p, st);
+  }
+  if (bf16) return launch_g32<__nv_bfloat16, 128>(xq, ldx, s_a, w, ldw, s_w, p, st);
+  return launch_g32<__half, 128>(xq, ldx, s_a, w, ldw, s_w, p, st);
 }
+

@@ -1140,6 +1140,26 @@ def test_bounded_wait_runs_out_and_is_reported(cuda_dev):
     run_gemm_case(cuda_dev, 2049, 768, 384, lowrank=False, bias=True, seed=6)
 
 
+
+@pytest.mark.parametrize("variant", [0, 1, 2])
+@pytest.mark.parametrize("M,K,N", [(1, 128, 4), (127, 256, 60), (129, 128, 68), (300, 384, 1096), (260, 640, 132)])
+def test_gemm_g32_tile_widths(cuda_dev, M, K, N, variant):
+    """Both tile widths of the group-32 GEMM (and the choice by size) at the edges of their tiles and on ragged outputs."""
+    g = torch.Generator().manual_seed(M + K + N)
+    x = torch.randn(M, K, generator=g).to(torch.float16)
+    w = torch.randn(N, K, generator=g) * 0.02
+    bias = torch.randn(N, generator=g) * 0.01
+    xq, sa = oracle.quant_rows_g32(x)
+    wq, sw = oracle.quant_rows_g32(w)
+    _lib.set_option("g32_variant", variant)
+    try:
+        y = int8_exec.int8_gemm_g32(xq.to(cuda_dev), sa.to(cuda_dev), wq.to(cuda_dev), sw.t().contiguous().to(cuda_dev),
+                                    bias.to(cuda_dev), torch.float16)
+    finally:
+        _lib.set_option("g32_variant", 0)
+    assert torch.equal(y.cpu(), oracle.gemm_g32(xq, sa, wq, sw, bias, torch.float16))
+
+
 # ------------------------------------------------------------------------------------------------ quantisation + down-projection
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,K,K1", [(1, 64, 0), (63, 128, 0), (64, 200, 0), (65, 1288, 0), (200, 1536, 0), (130, 1544, 0),
