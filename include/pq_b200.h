@@ -256,6 +256,26 @@ int pq_quant_rows_lowrank(const void* x0, int64_t K0, int64_t ldx0, const void* 
                           int64_t M, const void* a_t, int64_t lda, int R, int8_t* q, float* s, void* t, int64_t ldt,
                           void* workspace, size_t ws_bytes, void* stream);
 
+/* Whole forward of a Linear (quantisation, rank-32 down-projection, fused GEMM) from one descriptor of its constants:
+ * the launches of pq_quant_rows or pq_quant_rows_lowrank and of pq_int8_gemm, with the codes, t and row scales in `scratch`
+ * (256-byte aligned, pq_int8_linear_scratch_bytes; one per call in flight).  rank is 0 or 32; 32 needs 512 <= K <= 16384 and
+ * both lb [32, N] and its transpose lb_t [N, 32] as well as a_t [32, K], else PQ_ERR_UNSUPPORTED.  Int8Linear.forward,
+ * deploy/int8_exec.py:382-393. */
+typedef struct {
+  const int8_t* w; const float* s_col; const float* bias; const void* lb; const void* lb_t; const void* a_t;
+  int64_t ldw, ldb, N, K;
+  void* workspace; size_t ws_bytes;
+  int rank, dtype;
+} pq_linear_desc;
+int64_t pq_int8_linear_scratch_bytes(int64_t M, int64_t K, int rank);
+int pq_int8_linear(const pq_linear_desc* d, const void* x, int64_t ldx, int64_t M, void* scratch, int64_t scratch_bytes,
+                   void* out, int64_t ldo, void* stream);
+/* The same for a group-32 Linear: pq_quant_rows_g32 and pq_int8_gemm_g32. */
+int64_t pq_int8_linear_g32_scratch_bytes(int64_t M, int64_t K);
+int pq_int8_linear_g32(const void* x, int dtype, int64_t ldx, const int8_t* w, int64_t ldw, const float* s_w,
+                       const float* bias, void* scratch, int64_t scratch_bytes, void* out, int64_t ldo, int64_t M, int64_t N,
+                       int64_t K, void* workspace, size_t ws_bytes, void* stream);
+
 /* Low-tier weights at rest in 4 bits: expands packed nested-4-bit codes (pyraquant/quantizers_weight.py:182-199;
  * the reference keeps this tier for storage/BOPs accounting only, deploy/run_flux_latency.py:16-18) to the int8
  * operand the GEMMs read.  Byte b of row n holds element 2b in its low nibble and element 2b+1 in its high nibble,

@@ -68,6 +68,11 @@ SIGNATURES = {
     "pq_unpack_int4": (c_int, [c_void_p, c_int64, c_void_p, c_int64, c_int64, c_int64, c_void_p]),
     "pq_int8_gemm_g32": (c_int, [c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_void_p, c_void_p,
                                  c_void_p, c_int, c_int64, c_int64, c_int64, c_int64, c_void_p, c_size_t, c_void_p]),
+    "pq_int8_linear_scratch_bytes": (c_int64, [c_int64, c_int64, c_int]),
+    "pq_int8_linear": (c_int, [c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p]),
+    "pq_int8_linear_g32_scratch_bytes": (c_int64, [c_int64, c_int64]),
+    "pq_int8_linear_g32": (c_int, [c_void_p, c_int, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_void_p,
+                                   c_int64, c_int64, c_int64, c_int64, c_void_p, c_size_t, c_void_p]),
     "pq_scatter_rows": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
                                 c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p]),
     "pq_noalloc_scratch_bytes": (c_size_t, []),
@@ -77,6 +82,13 @@ SIGNATURES = {
     "pq_wait_probe": (c_int, [c_void_p, c_size_t, c_int, c_void_p]),
     "pq_i8_mma_issue_loop": (c_int, [c_int, c_int, c_void_p, c_void_p, c_size_t, c_void_p]),
 }
+
+
+class LinearDesc(ctypes.Structure):
+    """pq_linear_desc: a layer's constants for pq_int8_linear."""
+    _fields_ = [("w", c_void_p), ("s_col", c_void_p), ("bias", c_void_p), ("lb", c_void_p), ("lb_t", c_void_p), ("a_t", c_void_p),
+                ("ldw", c_int64), ("ldb", c_int64), ("N", c_int64), ("K", c_int64), ("workspace", c_void_p),
+                ("ws_bytes", c_size_t), ("rank", c_int), ("dtype", c_int)]
 
 
 def load() -> ctypes.CDLL:

@@ -20,6 +20,7 @@ Added entry points (not in the reference module): ``quant_rows_g32``, ``gather_q
 """
 from __future__ import annotations
 
+import ctypes
 import time
 from typing import Callable, Dict, Optional, Sequence, Tuple
 
@@ -301,6 +302,10 @@ class Int8Linear(nn.Module):
             self.lr_A = None
             self.lr_B = None
 
+    def __getstate__(self):
+        """Copies and pickles leave the address caches behind (they are remade on the first forward)."""
+        return {k: v for k, v in self.__dict__.items() if k != "_lean_cache"}
+
     def _lr_Bt(self) -> torch.Tensor:
         """K-major copy of lr_B for the tensor-core low-rank path, made once per device/dtype (not part of the state)."""
         return self._transposed("lr_B")
@@ -345,54 +350,52 @@ class Int8Linear(nn.Module):
                 and self.lr_A.dtype == x2.dtype and self.lr_B.dtype == x2.dtype and self.out_features % 8 == 0)
 
     def _lean_forward(self, x2: torch.Tensor):
-        """Eager fast path for the common case (aligned rows, rank-32 branch or none): the two C-ABI calls are made
-        straight from here with the per-layer constants cached, skipping the generic wrappers' checks.  Returns
-        None when the input does not qualify."""
+        """Eager fast path for the common case (aligned rows, no branch or a rank-32 one whose down-projection shares the
+        quantisation's launch): one C-ABI call with the per-layer constants in a descriptor, skipping the generic wrappers'
+        checks.  Returns None when the input does not qualify."""
         M, K = x2.shape
+        dt = x2.dtype
+        bufs = self._buffers
+        w = bufs["weight_int8"]
         if (M == 0 or not x2.is_cuda or x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16 or K % 16
-                or x2.device != self.weight_int8.device or x2.dtype not in ops._DT or torch.compiler.is_compiling()):
+                or x2.device != w.device or dt not in ops._DT or torch.compiler.is_compiling()):
             return None
-        lr = self.lr_A is not None
-        if lr and not self._fusable_lowrank(x2):
-            return None
-        c = self.__dict__.get("_lean_cache")
-        wptr = self.weight_int8.data_ptr()
+        lr_a = bufs.get("lr_A")
+        rank = 0
+        if lr_a is not None:
+            if not self._fusable_lowrank(x2) or not ops.quant_lowrank_ok(x2):
+                return None
+            rank = 32
+            lr_b, lbt, at = bufs["lr_B"], self._lr_Bt(), self._lr_At()
+            low = (lr_b.data_ptr(), lbt.data_ptr(), at.data_ptr())
+        else:
+            low = None
         # every buffer whose address is cached takes part in the key: .to(dtype) / .half() / load_state_dict(assign=True)
         # replace the float buffers while the int8 weight stays where it is
-        lbt = self._lr_Bt() if lr else None
-        key = (wptr, x2.dtype, self.w_scale.data_ptr(), self.bias.data_ptr() if self.bias is not None else 0,
-               self.lr_B.data_ptr() if lr else 0, lbt.data_ptr() if lr else 0)
+        sc, bias = bufs["w_scale"], bufs.get("bias")
+        key = (w.data_ptr(), dt, sc.data_ptr(), bias.data_ptr() if bias is not None else 0, low)
+        c = self.__dict__.get("_lean_cache")
         if c is None or c[0] != key:
-            assert self.w_scale.dtype == torch.float32 and (self.bias is None or self.bias.dtype == torch.float32), \
-                "w_scale and bias are fp32 buffers"
-            assert self.w_scale.numel() == self.out_features and (self.bias is None or self.bias.numel() == self.out_features)
-            c = (key, x2.dtype, self.weight_int8.stride(0), self.w_scale.data_ptr(),
-                 self.bias.data_ptr() if self.bias is not None else None,
-                 self.lr_B.data_ptr() if lr else None, self.lr_B.stride(0) if lr else 0,
-                 lbt.data_ptr() if lr else None, ops._DT[x2.dtype], ops._LIB(), ops.status_word(x2.device))
+            N = self.out_features
+            assert sc.dtype == torch.float32 and (bias is None or bias.dtype == torch.float32), "w_scale and bias are fp32 buffers"
+            assert sc.numel() == N and (bias is None or bias.numel() == N)
+            assert w.dtype == torch.int8 and w.stride(1) == 1 and K == w.shape[1], (w.shape, K)
+            ws = ops.status_word(x2.device)
+            d = ops._lib.LinearDesc(w=w.data_ptr(), s_col=sc.data_ptr(), bias=bias.data_ptr() if bias is not None else None,
+                                    lb=low[0] if low else None, lb_t=low[1] if low else None, a_t=low[2] if low else None,
+                                    ldw=w.stride(0), ldb=lr_b.stride(0) if low else 0, N=N, K=K, workspace=ws.data_ptr(),
+                                    ws_bytes=ws.numel() * 4, rank=rank, dtype=ops._DT[dt])
+            # the library, the descriptor and its address, and what the addresses in it belong to
+            c = (key, ops._LIB().pq_int8_linear, d, ctypes.addressof(d), N, K, ws)
             self.__dict__["_lean_cache"] = c
-        _w, _dt_t, ldw, sc_ptr, b_ptr, lb_ptr, ldb, lbt_ptr, code, lib, ws = c
-        N = self.out_features
-        dev = x2.device
-        t_ptr = None
-        ldt = 0
-        if lr:
-            q, sx, t = self._quant_down(x2)                     # t [M, 32]
-            t_ptr, ldt = t.data_ptr(), t.stride(0)
-        else:
-            q = torch.empty((M, K), dtype=torch.int8, device=dev)
-            sx = torch.empty((M,), dtype=torch.float32, device=dev)
-        out = torch.empty((M, N), dtype=x2.dtype, device=dev)
-        stream = ops._stream(x2)
+        _key, call, _d, d_ptr, N, K_w, _ws = c
+        assert K == K_w, (K, K_w)
+        nbytes = ops.linear_scratch_bytes(M, K, rank)
+        scratch = x2.new_empty((nbytes,), dtype=torch.uint8)
+        out = x2.new_empty((M, N))
         with ops._on_device(x2):
-            rc = 0
-            if not lr:
-                rc = lib.pq_quant_rows(x2.data_ptr(), code, M, K, x2.stride(0) if M > 1 else K, q.data_ptr(), sx.data_ptr(),
-                                       stream)
-            if rc == 0:
-                rc = lib.pq_int8_gemm(q.data_ptr(), K, sx.data_ptr(), wptr, ldw, sc_ptr, b_ptr, t_ptr, ldt, lb_ptr, ldb,
-                                      lbt_ptr, 32 if lr else 0, code, out.data_ptr(), code, N, M, N, K, ws.data_ptr(),
-                                      ws.numel() * 4, None, stream)
+            rc = call(d_ptr, x2.data_ptr(), x2.stride(0) if M > 1 else K, M, scratch.data_ptr(), nbytes, out.data_ptr(), N,
+                      ops._stream(x2))
         if rc:
             ops._lib.check(rc, f"Int8Linear(M={M}, N={N}, K={K})")
         return out
@@ -578,12 +581,13 @@ class Int8Linear(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         shape = x.shape
-        x2 = x.reshape(-1, shape[-1])
-        y = self._shared_forward(x2)
+        flat = len(shape) == 2
+        x2 = x if flat else x.reshape(-1, shape[-1])
+        y = self._shared_forward(x2) if "_shared_input" in self.__dict__ else None
         if y is None:
             y = self._lean_forward(x2)
         if y is not None:
-            return y.reshape(*shape[:-1], self.out_features)
+            return y if flat else y.reshape(*shape[:-1], self.out_features)
         if x2.stride(1) != 1:
             x2 = x2.contiguous()
         if self._fusable_lowrank(x2):
@@ -675,6 +679,10 @@ class Int8LinearG32(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         shape = x.shape
         x2 = x.reshape(-1, shape[-1])
+        if _eager():
+            y = ops.linear_g32(x2, self.weight_int8, self.w_scale_gm, self.bias)
+            if y is not None:
+                return y.reshape(*shape[:-1], self.out_features)
         xq, sa = quant_rows_g32(x2)
         y = int8_gemm_g32(xq, sa, self.weight_int8, self.w_scale_gm, self.bias, x2.dtype)
         return y.reshape(*shape[:-1], self.out_features)

@@ -318,6 +318,37 @@ def quant_rows_lowrank(x2: Tensor, a_t: Tensor, x_more: Optional[Tensor] = None)
     return q, s, t
 
 
+def linear_scratch_bytes(M: int, K: int, rank: int) -> int:
+    """pq_int8_linear_scratch_bytes, computed here (a call through ctypes costs as much as the arithmetic saves)."""
+    up = lambda v: (v + 255) & ~255
+    return up(M * K) + up(2 * M * rank) + up(4 * M)
+
+
+def linear_g32(x2: Tensor, w_int8: Tensor, s_w_gm: Tensor, bias: Optional[Tensor]) -> Optional[Tensor]:
+    """Quantisation and group-32 GEMM in one call (pq_int8_linear_g32); None when an operand is not as the kernels take it."""
+    M, K = x2.shape
+    N = w_int8.shape[0]
+    if (M == 0 or x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16 or K % 128 or K > 16384 or N % 4
+            or x2.dtype not in _DT or not x2.is_cuda or w_int8.device != x2.device or w_int8.shape[1] != K
+            or not w_int8.is_contiguous() or w_int8.dtype != torch.int8 or s_w_gm.dtype != torch.float32
+            or s_w_gm.shape != (K // 32, N) or not s_w_gm.is_contiguous()
+            or (bias is not None and (bias.dtype != torch.float32 or bias.numel() != N or not bias.is_contiguous()))):
+        return None
+    ng = (M * (K // 32) * 4 + 255) & ~255
+    nbytes = ((M * K + 255) & ~255) + ng
+    scratch = x2.new_empty((nbytes,), dtype=torch.uint8)
+    out = x2.new_empty((M, N))
+    ws = status_word(x2.device)
+    code = _DT[x2.dtype]
+    with _on_device(x2):
+        rc = _LIB().pq_int8_linear_g32(x2.data_ptr(), code, x2.stride(0) if M > 1 else K, w_int8.data_ptr(), K, s_w_gm.data_ptr(),
+                                       _ptr(bias), scratch.data_ptr(), nbytes, out.data_ptr(), N, M, N, K, ws.data_ptr(),
+                                       _lib.GEMM_WORKSPACE_BYTES, _stream(x2))
+    if rc:
+        _lib.check(rc, f"pq_int8_linear_g32(M={M}, N={N}, K={K})")
+    return out
+
+
 # ------------------------------------------------------------------------------------------------ 4-bit storage
 def pack_int4(codes: Tensor) -> Tensor:
     """int8 codes in [-8, 7], shape [N, K] with K even -> uint8 [N, K/2]: element 2b in the low nibble of byte b,

@@ -1194,3 +1194,29 @@ def test_quant_rows_lowrank(cuda_dev, M, K, K1, dtype):
     if Kt >= 512 and not K1:
         assert torch.equal(t, ops.lowrank_down(x0, a_t))              # the same slices, summed in the same order
         assert torch.equal(t[: M // 2], ops.quant_rows_lowrank(x0[: M // 2], a_t)[2])   # whatever the number of rows
+
+
+# ------------------------------------------------------------------------------------------------ whole forward in one call
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,N,lowrank", [(1, 64, 8, False), (154, 640, 1280, False), (77, 1808, 2376, False),
+                                           (33, 512, 264, True), (700, 3072, 512, True)])
+def test_linear_in_one_call(cuda_dev, M, K, N, lowrank, dtype):
+    """`Int8Linear.forward` through the one-call entry point == the separate operators, bit for bit; also on a row-strided
+    view, after a copy of the module, and after its scale buffer was replaced."""
+    import copy
+    g = torch.Generator().manual_seed(M + K + N)
+    m = _toy_layer(cuda_dev, g, K, N, lowrank=lowrank, dtype=dtype)
+    wide = rand_act(M, K + 24, dtype, M + 7).to(cuda_dev)
+    for x in (wide[:, :K].contiguous(), wide[:, :K]):
+        y = m(x)
+        assert "_lean_cache" in m.__dict__
+        xq, sx = int8_exec.quant_rows(x)
+        if lowrank:
+            want = int8_exec.int8_gemm_lr(xq, sx, m.weight_int8, m.w_scale, m.bias, m._down(x), m.lr_B, dtype)
+        else:
+            want = int8_exec.int8_gemm_fused(xq, sx, m.weight_int8, m.w_scale, m.bias, dtype)
+        assert torch.equal(y, want)
+    c = copy.deepcopy(m)
+    assert torch.equal(c(x), want)
+    c.w_scale = c.w_scale * 2
+    assert torch.equal(m(x), want) and not torch.equal(c(x), want)
