@@ -516,6 +516,22 @@ int choose_block_n(int64_t M, int64_t N) {
   return 256;
 }
 
+// CTA-pair tiles (256 x 256 on two SMs) or single-CTA ones.  A k-block of a 128 x 128 tile brings in 32 KB for 256 cycles
+// of MMA, one of a pair tile 32 KB per SM for 512: both take the 512 cycles that 32 KB need at the 64 bytes per clock an SM
+// gets from L2, so what counts is the number of tiles an SM goes through, padding included.  Measured (pair / single, us):
+// 3001 x 1808 -> 2376 (2 against 4 tiles) 20.2 / 31, 30000 x 320 -> 320 (4 / 5) 12.8 / 24.6, 65536 x 640 -> 640 (11 / 18)
+// 34.7 / 38.8, 1024 x 12288 -> 3072 rank 32 (1 / 2) 37.4 / 43.8, 700 x 3072 -> 9216 rank 32 (2 / 3) 24.3 / 24.4, and where a
+// short K leaves the longer epilogue of the wide tile exposed 4096 x 640 -> 640 (1 / 2) 8.0 / 7.3.
+bool prefer_pair(int bn, int64_t pair_rows, int64_t M, int64_t N, int64_t K, bool has_lr) {
+  const int64_t pair_tiles = pair_rows * ((N + 255) / 256), pairs = sm_count() / 2;
+  if (bn == 256 && pair_tiles >= pairs) return true;
+  if (options().gemm_block_n != 0) return false;
+  const int64_t pair_steps = (pair_tiles + pairs - 1) / pairs;
+  const int64_t single_steps = (((M + BM - 1) / BM) * ((N + 127) / 128) + sm_count() - 1) / sm_count();
+  if (pair_steps == 1) return single_steps >= 3 || (single_steps == 2 && K >= 2048);
+  return has_lr ? 5 * single_steps >= 8 * pair_steps : single_steps > pair_steps;
+}
+
 int gemm_common(const int8_t* xq, int64_t ldx, const float* s_row, const int8_t* w0, const float* sc0,
                 const int8_t* w1, const float* sc1, int64_t ldw, const float* bias, const void* t, int64_t ldt,
                 const void* lb, int64_t ldb, const void* lb_t, int R, int lr_dtype, void* out, int out_dtype,
@@ -579,8 +595,8 @@ int gemm_common(const int8_t* xq, int64_t ldx, const float* s_row, const int8_t*
       return launch_gemm_pair(out_dtype == PQ_DTYPE_BF16, dbg_acc != nullptr || p.timing != nullptr, xq, ldx, w0, w1, ldw, has_lr ? t : nullptr, ldt,
                               has_lr ? lb_t : nullptr, M, N, K, p, static_cast<cudaStream_t>(stream));
     }
-    if (options().gemm_pair != 0 && bn == 256 && pair_legal &&
-        pair_rows * ((N + 255) / 256) >= (options().gemm_pair == 2 ? 1 : sm_count() / 2)) {
+    const bool want_pair = options().gemm_pair == 2 ? bn == 256 : prefer_pair(bn, pair_rows, M, N, K, has_lr);
+    if (options().gemm_pair != 0 && pair_legal && want_pair) {
       return launch_gemm_pair(out_dtype == PQ_DTYPE_BF16, dbg_acc != nullptr || p.timing != nullptr, xq, ldx, w0, w1, ldw, has_lr ? t : nullptr, ldt,
                               has_lr ? lb_t : nullptr, M, N, K, p, static_cast<cudaStream_t>(stream));
     }

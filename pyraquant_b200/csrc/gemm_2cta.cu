@@ -30,24 +30,30 @@ constexpr int kLrChunks = 2;               // the low-rank term is added in colu
 constexpr int kLrChunkN = PBN / kLrChunks; // 128 columns: one kind::f16 MMA pair per chunk
 constexpr int kLbChunkRows = kLrChunkN / 2;   // lbT rows each CTA stages per chunk
 // Warps of a CTA: 0 TMA producer, 1 MMA issuer, 2 .. 2 + EW - 1 epilogue, 2 + EW issuer of the low-rank MMAs (leader
-// CTA).  EW = 8 when the main loop of a tile outlasts its epilogue (long K); EW = 16 for short K without a low-rank
-// term, where the epilogue is the critical path: each warp then owns 16 rows x 128 columns instead of 32 x 128.
+// CTA).  EW = 8 when the main loop of a tile outlasts its epilogue (long K); EW = 16 where the epilogue is the critical path:
+// each warp then owns 16 rows x 128 columns (with a low-rank term) or 32 x 64 instead of 32 x 128.
 constexpr int pair_threads(int ew) { return (3 + ew) * 32; }
-constexpr int kShortK = 1536;              // up to this K (and without a low-rank term) the sixteen-warp epilogue is used
+constexpr int kShortK = 2048;              // up to this K the sixteen-warp epilogue is used,
+constexpr int kFewBlocks = 160;            // and up to this many k-blocks per pair
 
+// WIDE: the sixteen-warp epilogue without low-rank term, whose output tiles leave through shared memory: one operand stage
+// less (short K needs few), two 2 KB staging blocks per epilogue warp where the t / lbT tiles of the other form are.
+template <bool WIDE>
 struct PairSmem {
+  static constexpr int kStages = WIDE ? PSTAGES - 1 : PSTAGES;
   static constexpr int kABytes = BM * BK;
   static constexpr int kBBytes = kHalfB * BK;
   static constexpr int kStageBytes = kABytes + kBBytes;            // per CTA
-  static constexpr int kTOff = PSTAGES * kStageBytes;
+  static constexpr int kTOff = kStages * kStageBytes;
   static constexpr int kTBytes = BM * kRowBytesLr;                 // per CTA: its 128 rows of t
   static constexpr int kLbOff = kTOff + 2 * kTBytes;
   static constexpr int kLbBytes = kHalfB * kRowBytesLr;            // per CTA: its 128 rows of lbT
-  static constexpr int kScolOff = kLbOff + 2 * kLbBytes;            // two lbT buffers: consecutive column tiles alternate
+  static constexpr int kStageBlock = 16 * 64 * 2;                  // 16 rows x 64 columns of output
+  static constexpr int kScolOff = WIDE ? kTOff + 16 * 2 * kStageBlock : kLbOff + 2 * kLbBytes;   // two lbT buffers: consecutive column tiles alternate
   static constexpr int kBiasOff = kScolOff + PBN * 4;
   static constexpr int kBarOff = kBiasOff + PBN * 4;
   // full[S], empty[S], tfull[2], tempty[2], t_full[2], lb_full[2], ylr_ready[2][chunks], lr_done[2][chunks]
-  static constexpr int kNumBars = 2 * PSTAGES + 8 + 4 * kLrChunks;
+  static constexpr int kNumBars = 2 * kStages + 8 + 4 * kLrChunks;
   static constexpr int kMiscOff = kBarOff + kNumBars * 8;
   static constexpr int kTotal = kMiscOff + 16 + 64;      // + time stamps of the cycle-counter experiments
   static_assert(kTotal <= 232448, "exceeds the 227 KB shared memory of one CTA");
@@ -247,13 +253,15 @@ __global__ void __launch_bounds__(pair_threads(EW), 1)
 pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmW,
                                const __grid_constant__ CUtensorMap tmW1, const __grid_constant__ CUtensorMap tmT, const __grid_constant__ CUtensorMap tmLbT,
                                const __grid_constant__ CUtensorMap tmOut, const GemmParams p) {
-  using L = PairSmem;
+  constexpr bool WIDE = EW == 16 && !HAS_LR;
+  using L = PairSmem<WIDE>;
+  constexpr int kStages = L::kStages;
   static_assert(EW == 8 || EW == 16, "eight or sixteen epilogue warps");
   constexpr int kLrWarp = 2 + EW;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
-  uint64_t* empty_bar = full_bar + PSTAGES;
-  uint64_t* tfull_bar = empty_bar + PSTAGES;
+  uint64_t* empty_bar = full_bar + kStages;
+  uint64_t* tfull_bar = empty_bar + kStages;
   uint64_t* tempty_bar = tfull_bar + 2;
   uint64_t* t_full = tempty_bar + 2;
   uint64_t* lb_full = t_full + 2;
@@ -282,7 +290,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmW1);
     if (HAS_LR) { tma_prefetch_desc(&tmT); tma_prefetch_desc(&tmLbT); }
-    for (int s = 0; s < PSTAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 2 * EW);
       mbar_init(&t_full[b], 1);
@@ -355,7 +363,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
           if (p.l2_hints & 1) tma_load_2d_pair_hint(a_s + L::kABytes, wm, fb, kb * BK, nhalf0, pol_w);
           else tma_load_2d_pair(a_s + L::kABytes, wm, fb, kb * BK, nhalf0);
           ++issued;
-          if (++stage == PSTAGES) { stage = 0; phase ^= 1u; }
+          if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
         if (HAS_LR) {
@@ -369,9 +377,9 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
       }
       // copies in flight must land before the CTA may exit: the last stages issued are consumed by MMAs whose
       // completion is committed to this CTA's empty barriers
-      const int pending = issued < PSTAGES ? static_cast<int>(issued) : PSTAGES;
+      const int pending = issued < kStages ? static_cast<int>(issued) : kStages;
       for (int i = 0; i < pending; ++i) {
-        if (--stage < 0) { stage = PSTAGES - 1; phase ^= 1u; }
+        if (--stage < 0) { stage = kStages - 1; phase ^= 1u; }
         if (!wait_or_abort(&empty_bar[stage], phase, abort_flag)) {
           for (int k = 0; k < 64; ++k) __nanosleep(1000);
           break;
@@ -417,7 +425,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
             tc_mma_i8_pair(d_tmem, a_desc + static_cast<uint64_t>(2 * k), b_desc + static_cast<uint64_t>(2 * k), idesc,
                            (kb > 0 || k > 0) ? 1u : 0u);
           commit_both(&empty_bar[stage]);
-          if (++stage == PSTAGES) { stage = 0; phase ^= 1u; }
+          if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
         commit_both(&tfull_bar[buf]);
@@ -469,9 +477,12 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
     // ------------------------------------------------------------------ epilogue (warps 2 .. 2 + EW - 1 of both CTAs)
     const int quarter = warp & 3;
     const int half = ((warp - 2) >> 2) & 1;
-    // sixteen warps: warps 2..9 take the first 16 rows of each 32-row lane quarter, warps 10..17 the other 16
-    constexpr int MBN = EW == 16 ? 1 : 2;                // 16-row blocks per warp
-    const int mb_base = EW == 16 ? ((warp - 2) >> 3) : 0;
+    // Sixteen warps with a low-rank term: warps 2..9 take the first 16 rows of each 32-row lane quarter, warps 10..17 the
+    // other 16, of every chunk.  Without one (WIDE) a warp takes all 32 rows of 64 columns, so that the column scales and
+    // the bias of its columns are read from shared memory once per tile.
+    constexpr int MBN = EW == 16 && !WIDE ? 1 : 2;       // 16-row blocks per warp
+    const int mb_base = EW == 16 && !WIDE ? ((warp - 2) >> 3) : 0;
+    const int colg = (warp - 2) >> 2;                    // WIDE: columns [64 colg, +64) of the tile
     const int etid = threadIdx.x - 64;
     const int g = lane >> 2, q = lane & 3;
     constexpr int UNIT_N = 64;
@@ -480,6 +491,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
     float* scol_s = reinterpret_cast<float*>(smem + L::kScolOff);
     float* bias_s = reinterpret_cast<float*>(smem + L::kBiasOff);
     const bool vec_store = (p.ldo % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.out) & 15) == 0);
+    const bool gelu = (p.epi_flags & PQ_EPI_GELU_TANH) != 0;
     bool aborted = false;
     int it = 0;
     int aux_n0 = -1, aux_set = -1;
@@ -519,9 +531,13 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
       }
       // row scales of this tile: fetched while the previous tile was being stored (first tile: here)
       float srow[2][2];
-      if (it == 0) load_srow(c, srow_next);
+      if constexpr (WIDE) {
+        load_srow(c, srow);                              // on its way while this warp waits for the accumulator
+      } else {
+        if (it == 0) load_srow(c, srow_next);
 #pragma unroll
-      for (int mb = 0; mb < MBN; ++mb) { srow[mb][0] = srow_next[mb][0]; srow[mb][1] = srow_next[mb][1]; }
+        for (int mb = 0; mb < MBN; ++mb) { srow[mb][0] = srow_next[mb][0]; srow[mb][1] = srow_next[mb][1]; }
+      }
 
       const long long e1 = timing ? clock64() : 0;
       if (!aborted) {
@@ -533,14 +549,15 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
       if (trace && it < 1000 && warp == 2 && lane == 0) trace[it * 24 + 20 + rank] = static_cast<long long>(global_timer_ns());
       const long long e2 = timing ? clock64() : 0;
       long long e3 = e2, e4 = e2;
-      {
+      if constexpr (!WIDE) {
         PairWalker wn = w; wn.advance();
         if (wn.valid()) load_srow(pair_coord(wn.mt, mt0, p, rank), srow_next);
       }
 
       // Column assignment: chunk ch of the tile is columns [ch * 128, +128); the warps of half 0 take its first 64
       // columns, those of half 1 the other 64, so that one low-rank MMA pair per chunk serves all sixteen warps.
-      const uint32_t t_acc = tmem_base + static_cast<uint32_t>(buf * PBN + half * UNIT_N);
+      const uint32_t t_acc = tmem_base + static_cast<uint32_t>(buf * PBN + (WIDE ? colg : half) * UNIT_N);
+      auto col_unit_of = [&](int ch) { return WIDE ? colg * UNIT_N : ch * kLrChunkN + half * UNIT_N; };
       auto unit_addr = [&](int ch, int mb) {
         return t_acc + (static_cast<uint32_t>(quarter * 32 + (mb_base + mb) * 16) << 16) + static_cast<uint32_t>(ch * kLrChunkN);
       };
@@ -548,7 +565,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
 
       // scale one 16 x 64 block: int32 -> fp32 * (s_row * s_col), in place in the registers
       auto scale_unit = [&](uint32_t (&v)[32], int ch, int mb) {
-        const int col_unit = ch * kLrChunkN + half * UNIT_N;
+        const int col_unit = col_unit_of(ch);
         const float2 srA = make_float2(srow[mb][0], srow[mb][0]), srB = make_float2(srow[mb][1], srow[mb][1]);
 #pragma unroll
         for (int nb = 0; nb < 8; ++nb) {
@@ -568,7 +585,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
       };
       // + bias, round, transpose inside quads, store one 16 x 64 block of fp32 values
       auto store_unit = [&](const uint32_t (&v)[32], int ch, int mb) {
-        const int col_unit = ch * kLrChunkN + half * UNIT_N;
+        const int col_unit = col_unit_of(ch);
         const int rA = row0 + quarter * 32 + (mb_base + mb) * 16 + g;
         const int rB = rA + 8;
 #pragma unroll
@@ -667,30 +684,60 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
         }
       };
 
-      // Sixteen-warp tiles without low-rank term are bound by the integer pipe and the global-store path: the rounded
-      // 16 x 64 block goes to shared memory in the 128-byte-swizzled layout (conflict-free: the eight rows of a store
-      // land in eight different 16-byte columns) and one TMA store writes it; no in-quad transposes, no row
-      // predicates (TMA clips at M and N).  The staging buffers are the t / lbT tiles this variant does not use.
-      auto stage_unit = [&](const uint32_t (&v)[32], int ch) {
-        const int col_unit = ch * kLrChunkN + half * UNIT_N;
-        uint8_t* sbuf = smem + L::kTOff + (warp - 2) * 2048;
-        if (lane == 0) bulk_wait_group_read0();            // the previous store of this warp has read the buffer
+      // WIDE tiles of a plain call go out through shared memory: a warp's rounded 32 x 64 block in the 128-byte-swizzled
+      // layout, one TMA store each (TMA clips at M and N).  No in-quad transposes, row predicates or flag tests per store,
+      // the hardware conversion instead of five instructions, the column data read once per tile, and the accumulator
+      // handed back as soon as it is in registers.  65536 x 640 -> 5120 fp16 264 -> 237 us, 671 MB of output that a plain
+      // fill takes 173 us for; 8.6 instead of 14.2 warp instructions per element.  What is left is the store path: the
+      // same time with two groups of eight warps alternating tiles, and 271 us with one thread issuing all stores.
+      auto staged_tile = [&](auto act) {                     // act: with the GELU (two copies, so that neither carries the other's code)
+        uint32_t v0[16], v1[16];
+        uint8_t* const blk = smem + L::kTOff + (warp - 2) * 2 * L::kStageBlock;     // rows 0-15, then rows 16-31
+        uint8_t* const mine = blk + g * 128 + q * 4;
+        tmem_ld_16x256b_x4(unit_addr(0, 0), v0);
+        if (lane == 0) bulk_wait_group_read0();              // the previous tile's stores have read the two blocks
         __syncwarp();
 #pragma unroll
-        for (int nb = 0; nb < 8; ++nb) {
-          const float2 bi = *reinterpret_cast<const float2*>(bias_s + col_unit + nb * 8 + 2 * q);
-          uint32_t wA = pack2(__fadd_rn(__uint_as_float(v[4 * nb + 0]), bi.x), __fadd_rn(__uint_as_float(v[4 * nb + 1]), bi.y), OutT{});
-          uint32_t wB = pack2(__fadd_rn(__uint_as_float(v[4 * nb + 2]), bi.x), __fadd_rn(__uint_as_float(v[4 * nb + 3]), bi.y), OutT{});
-          if (p.epi_flags & PQ_EPI_GELU_TANH) { wA = gelu_word<OutT>(wA); wB = gelu_word<OutT>(wB); }
-          uint8_t* dst = sbuf + g * 128 + ((nb ^ g) << 4) + q * 4;
-          st_shared_u32(dst, wA);
-          st_shared_u32(dst + 8 * 128, wB);                // row g + 8: same swizzle phase
+        for (int hc = 0; hc < 2; ++hc) {                     // 32 columns, both 16-row blocks
+          float2 sc[4], bi[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            sc[j] = *reinterpret_cast<const float2*>(scol_s + colg * UNIT_N + (hc * 4 + j) * 8 + 2 * q);
+            bi[j] = *reinterpret_cast<const float2*>(bias_s + colg * UNIT_N + (hc * 4 + j) * 8 + 2 * q);
+          }
+#pragma unroll
+          for (int mb = 0; mb < 2; ++mb) {
+            uint32_t (&v)[16] = mb == 0 ? v0 : v1;
+            tc_wait_ld();
+            if (mb == 0) tmem_ld_16x256b_x4(unit_addr(0, 1) + hc * 32, v1);
+            else if (hc == 0) tmem_ld_16x256b_x4(unit_addr(0, 0) + 32, v0);
+            if (mb == 1 && hc == 1) {                        // everything is in registers: the accumulator is free
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster(leader_addr(&tempty_bar[buf]));
+            }
+            const float2 srA = make_float2(srow[mb][0], srow[mb][0]), srB = make_float2(srow[mb][1], srow[mb][1]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float2 pA = make_float2(__int2float_rn(static_cast<int32_t>(v[4 * j + 0])), __int2float_rn(static_cast<int32_t>(v[4 * j + 1])));
+              const float2 pB = make_float2(__int2float_rn(static_cast<int32_t>(v[4 * j + 2])), __int2float_rn(static_cast<int32_t>(v[4 * j + 3])));
+              const float2 yA = __fmul2_rn(pA, __fmul2_rn(srA, sc[j])), yB = __fmul2_rn(pB, __fmul2_rn(srB, sc[j]));
+              // scalar additions: packed ones, even written as add.rn.f32x2, get contracted with the products
+              uint32_t wA = pack2(__fadd_rn(yA.x, bi[j].x), __fadd_rn(yA.y, bi[j].y), OutT{});
+              uint32_t wB = pack2(__fadd_rn(yB.x, bi[j].x), __fadd_rn(yB.y, bi[j].y), OutT{});
+              if constexpr (decltype(act)::value) { wA = gelu_word<OutT>(wA); wB = gelu_word<OutT>(wB); }
+              // 16-byte column nb of row g sits at nb ^ g (128-byte swizzle): the eight rows of a store hit different banks
+              uint8_t* dst = mine + mb * L::kStageBlock + (((hc * 4 + j) ^ g) << 4);
+              st_shared_u32(dst, wA);
+              st_shared_u32(dst + 8 * 128, wB);              // row g + 8: same swizzle phase
+            }
+          }
         }
         fence_proxy_async_smem();
         __syncwarp();
-        const int r_first = row0 + quarter * 32 + mb_base * 16;
-        if (lane == 0 && r_first < row_end && n0 + col_unit < p.N) {
-          tma_store_2d(&tmOut, sbuf, n0 + col_unit, r_first);
+        const int r_first = row0 + quarter * 32;             // one box of 32 rows: its two blocks are neighbours
+        if (lane == 0 && r_first < row_end && n0 + colg * UNIT_N < p.N) {
+          tma_store_2d(&tmOut, blk, n0 + colg * UNIT_N, r_first);
           bulk_commit_group();
         }
       };
@@ -738,18 +785,25 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
         }
         return true;
       };
+      if (WIDE && !DBG && p.tma_store) {
+        if (gelu) staged_tile(std::true_type{});
+        else staged_tile(std::false_type{});
+        continue;                                          // it has handed the accumulator back
+      } else {
       if (!chunk_ready(0)) { aborted = true; continue; }
       tmem_ld_16x256b_x8(unit_addr(0, 0), va);
 #pragma unroll 1
-      for (int ch = 0; ch < kLrChunks; ++ch) {
+      for (int ch = 0; ch < (WIDE ? 1 : kLrChunks); ++ch) {
         tc_wait_ld();
-        if constexpr (EW == 16) {                         // one 16-row block per warp and chunk; the other warps overlap
-          if constexpr (!HAS_LR) scale_unit(va, ch, 0);
-          bool staged = false;
-          if constexpr (!HAS_LR) {
-            if (p.tma_store) { stage_unit(va, ch); staged = true; }
-          }
-          if (!staged) store_unit(va, ch, 0);
+        if constexpr (WIDE) {                             // both 16-row blocks of the warp's columns, one after the other
+          scale_unit(va, ch, 0);
+          store_unit(va, ch, 0);
+          tmem_ld_16x256b_x8(unit_addr(ch, 1), va);
+          tc_wait_ld();
+          scale_unit(va, ch, 1);
+          store_unit(va, ch, 1);
+        } else if constexpr (EW == 16) {                  // one 16-row block per warp and chunk; the other warps overlap
+          store_unit(va, ch, 0);
           if (ch + 1 < kLrChunks) {
             if (!chunk_ready(ch + 1)) { aborted = true; break; }
             tmem_ld_16x256b_x8(unit_addr(ch + 1, 0), va);
@@ -767,6 +821,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
           store_unit(vb, ch, 1);
         }
       }
+      }
       if (aborted) continue;
       e4 = e3 + lr_wait;
       tc_fence_before();
@@ -774,7 +829,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
       if (lane == 0) mbar_arrive_cluster(leader_addr(&tempty_bar[buf]));
       if (timing) { te_aux += e1 - e0; te_tfull += e2 - e1; te_p1 += e3 - e2; te_lr += e4 - e3; te_p2 += clock64() - e4; }
     }
-    if (EW == 16 && !HAS_LR && p.tma_store && lane == 0) bulk_wait_group0();   // stores done before shared memory goes
+    if (WIDE && p.tma_store && lane == 0) bulk_wait_group0();   // stores done before shared memory goes
     if (timing && warp == 2 && lane == 0) {
       timing[blockIdx.x * 16 + 2] = te_aux; timing[blockIdx.x * 16 + 3] = te_tfull; timing[blockIdx.x * 16 + 4] = te_p1;
       timing[blockIdx.x * 16 + 5] = te_lr; timing[blockIdx.x * 16 + 6] = te_p2; timing[blockIdx.x * 16 + 7] = it;
@@ -794,13 +849,13 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
   }
 }
 
-// Output [M, N] of 16-bit elements, row stride ldo: boxes of 64 columns x 16 rows, 128-byte swizzle (TMA store).
+// Output [M, N] of 16-bit elements, row stride ldo: boxes of 64 columns x 32 rows, 128-byte swizzle (TMA store).
 int make_out_map16(CUtensorMap* map, void* base, int64_t M, int64_t N, int64_t ldo, bool bf16) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return PQ_ERR_CUDA;
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(M)};
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(ldo) * 2};
-  cuuint32_t box[2] = {64, 16};
+  cuuint32_t box[2] = {64, 32};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides,
                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
@@ -815,7 +870,7 @@ int launch_pair_ew(const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtenso
   // sixteen-warp tiles of a plain single-tier call store through shared memory + TMA when the output allows it
   CUtensorMap tmOut = tmA;
   p.tma_store = 0;
-  if (EW == 16 && !HAS_LR && p.m_split == p.M && !(p.epi_flags & (PQ_EPI_ACCUMULATE | PQ_EPI_GATE)) && p.n_out_more == 0 && options().gemm_tma_store != 0 &&
+  if (EW == 16 && !HAS_LR && !DBG && p.m_split == p.M && !(p.epi_flags & (PQ_EPI_ACCUMULATE | PQ_EPI_GATE)) && p.n_out_more == 0 && options().gemm_tma_store != 0 &&
       p.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0) {
     const int rc = make_out_map16(&tmOut, p.out, p.M, p.N, p.ldo, std::is_same<OutT, __nv_bfloat16>::value);
     if (rc != PQ_OK) return rc;
@@ -831,11 +886,11 @@ int launch_pair_ew(const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtenso
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.blockDim = dim3(pair_threads(EW), 1, 1);
-  cfg.dynamicSmemBytes = PairSmem::kTotal;
+  cfg.dynamicSmemBytes = PairSmem<EW == 16 && !HAS_LR>::kTotal;
   cfg.stream = st;
   cfg.attrs = attr; cfg.numAttrs = 1;
   if (max_pairs[dev] == 0) {
-    PQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::kTotal));
+    PQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<EW == 16 && !HAS_LR>::kTotal));
     cfg.gridDim = dim3(2 * sm_count(), 1, 1);
     int n = 0;
     PQ_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));
@@ -883,13 +938,19 @@ int launch_pair_ew(const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtenso
   return PQ_OK;
 }
 
-// Sixteen epilogue warps when the K loop of a tile is shorter than its epilogue and there is no low-rank term (measured:
-// 5-12 % faster there, slower with the two-pass low-rank epilogue); option gemm_epi_warps overrides (0 = this rule).
+// Sixteen epilogue warps where the epilogue shows: a short K (the main loop of a tile is over before its epilogue) and
+// launches of few k-blocks per pair, whose last tile's epilogue is a good part of the time.  In long launches, bound by power
+// and not by the epilogue, the eight warps are ahead by 5-8 % (16896 x 3072 -> 12288: 389 / 427 us).  Eight / sixteen, us:
+// without low-rank term 2048 x 8192 -> 4096 56.3 / 50.5, 4608 x 5120 -> 1280 34.5 / 32.4, 16384 x 640 -> 640 24.4 / 13.1;
+// with it 16896 x 1536 -> 6144 171 / 150, 40000 x 1024 -> 2048 114 / 103, 3000 x 3072 -> 1344 21.0 / 19.2,
+// 4608 x 3072 -> 3072 33.6 / 32.8.  Option gemm_epi_warps overrides.
 template <typename OutT, bool HAS_LR, bool DBG>
 int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtensorMap& tmW1, const CUtensorMap& tmT,
                 const CUtensorMap& tmLbT, GemmParams p, int mt_pairs, int ntl, cudaStream_t st) {
   const int want = options().gemm_epi_warps;
-  const bool wide = want == 16 || (want != 8 && !HAS_LR && p.K <= kShortK);
+  const int64_t pairs = sm_count() / 2;
+  const int64_t kblocks = (static_cast<int64_t>(mt_pairs) * ntl + pairs - 1) / pairs * ((p.K + BK - 1) / BK);
+  const bool wide = want == 16 || (want != 8 && (p.K <= kShortK || kblocks <= kFewBlocks));
   if (wide) return launch_pair_ew<OutT, HAS_LR, DBG, 16>(tmA, tmW, tmW1, tmT, tmLbT, p, mt_pairs, ntl, st);
   return launch_pair_ew<OutT, HAS_LR, DBG, 8>(tmA, tmW, tmW1, tmT, tmLbT, p, mt_pairs, ntl, st);
 }

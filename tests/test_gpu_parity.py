@@ -287,6 +287,30 @@ def test_gemm_production_kernels_bit_equal_without_lowrank(cuda_dev, dtype):
         assert torch.equal(y.cpu(), y32), (pair, bn, ew)
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K,ew,pair", [(8192, 1288, 320, 16, 2), (3001, 2376, 1808, 0, 1), (30000, 320, 320, 0, 1), (257, 136, 128, 16, 2),
+                                           (2048, 1032, 2304, 8, 2)])
+def test_gemm_pair_epilogues_bit_equal_on_many_outputs(cuda_dev, dtype, M, N, K, ew, pair):
+    """Product and sum of the epilogue are rounded separately: a fused multiply-add shows in about one output of 100 000, so
+    millions of outputs are compared with torch's separate fp32 operations (the accumulators are exact in fp64 and below
+    2^24).  Ragged row and column tails of the tiles that leave through shared memory, and the choice of kernel by size."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    xq = torch.randint(-127, 128, (M, K), generator=g, device=cuda_dev, dtype=torch.int8)
+    wq = torch.randint(-127, 128, (N, K), generator=g, device=cuda_dev, dtype=torch.int8)
+    sr = torch.rand(M, generator=g, device=cuda_dev) * 0.05 + 0.001
+    sc = torch.rand(N, generator=g, device=cuda_dev) * 2e-4 + 1e-5
+    b = torch.randn(N, generator=g, device=cuda_dev) * 0.01
+    acc = (xq.double() @ wq.double().t())
+    assert acc.abs().max().item() < 2 ** 24
+    want = ((acc.float() * (sr[:, None] * sc[None, :])) + b[None, :]).to(dtype)
+    _lib.set_option("gemm_pair", pair); _lib.set_option("gemm_epi_warps", ew)
+    try:
+        y = int8_exec.int8_gemm_fused(xq, sr, wq, sc, b, dtype)
+    finally:
+        _lib.set_option("gemm_pair", 1); _lib.set_option("gemm_epi_warps", 0)
+    assert torch.equal(y, want)
+
+
 @pytest.mark.parametrize("pair", [0, 2])
 def test_gemm_accumulators_beyond_24_bits_round_like_the_restatement(cuda_dev, pair):
     """Same-sign codes and K = 8192 give accumulators of 2^24 .. 2^27 with arbitrary low bits: the int32 -> fp32
