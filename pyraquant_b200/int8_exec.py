@@ -360,19 +360,21 @@ class Int8Linear(nn.Module):
         if (M == 0 or not x2.is_cuda or x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16 or K % 16
                 or x2.device != w.device or dt not in ops._DT or torch.compiler.is_compiling()):
             return None
-        lr_a = bufs.get("lr_A")
+        # absent ones are plain None attributes, and may have been set to a tensor since
+        attrs = self.__dict__
+        lr_a, bias = bufs.get("lr_A", attrs.get("lr_A")), bufs.get("bias", attrs.get("bias"))
         rank = 0
         if lr_a is not None:
             if not self._fusable_lowrank(x2) or not ops.quant_lowrank_ok(x2):
                 return None
             rank = 32
-            lr_b, lbt, at = bufs["lr_B"], self._lr_Bt(), self._lr_At()
+            lr_b, lbt, at = self.lr_B, self._lr_Bt(), self._lr_At()
             low = (lr_b.data_ptr(), lbt.data_ptr(), at.data_ptr())
         else:
             low = None
         # every buffer whose address is cached takes part in the key: .to(dtype) / .half() / load_state_dict(assign=True)
         # replace the float buffers while the int8 weight stays where it is
-        sc, bias = bufs["w_scale"], bufs.get("bias")
+        sc = bufs["w_scale"]
         key = (w.data_ptr(), dt, sc.data_ptr(), bias.data_ptr() if bias is not None else 0, low)
         c = self.__dict__.get("_lean_cache")
         if c is None or c[0] != key:

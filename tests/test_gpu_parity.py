@@ -1244,3 +1244,13 @@ def test_linear_in_one_call(cuda_dev, M, K, N, lowrank, dtype):
     assert torch.equal(c(x), want)
     c.w_scale = c.w_scale * 2
     assert torch.equal(m(x), want) and not torch.equal(c(x), want)
+    # a bias and a branch that are set as plain attributes of a layer made without them take part
+    if K % 32 == 0 and K >= 512 and N % 8 == 0:
+        bare = _toy_layer(cuda_dev, g, K, N, lowrank=False, bias=False, dtype=dtype)
+        bare.bias = torch.randn(N, generator=g).to(cuda_dev)
+        with_bias = bare(x)
+        assert torch.equal(with_bias, int8_exec.int8_gemm_fused(xq, sx, bare.weight_int8, bare.w_scale, bare.bias, dtype))
+        bare.lr_A = (torch.randn(K, 32, generator=g) * 0.05).to(dtype).to(cuda_dev)
+        bare.lr_B = (torch.randn(32, N, generator=g) * 0.05).to(dtype).to(cuda_dev)
+        assert torch.equal(bare(x), int8_exec.int8_gemm_lr(xq, sx, bare.weight_int8, bare.w_scale, bare.bias, bare._down(x),
+                                                           bare.lr_B, dtype))
