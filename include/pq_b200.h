@@ -300,6 +300,14 @@ int pq_scatter_rows(const void* y, int64_t ldy, int64_t M_act,
                     int64_t n_tokens, void* canvas, int64_t ldc, int64_t rows, int64_t C,
                     int dtype, void* stream);
 
+/* The same out of place (fuse_patch_predictions returns a new image, flux/routing.py:328-379): out gets the blended rows of
+ * the touched tokens and, for every row listed in rest [n_rest], the background's row unchanged.  tokens and rest together
+ * list every row once; background and out do not overlap.  One launch that moves each row once, instead of a copy of the
+ * background followed by pq_scatter_rows. */
+int pq_fuse_rows(const void* y, int64_t ldy, int64_t M_act, const int32_t* tokens, const int32_t* ptr, const int32_t* src,
+                 const float* beta, int64_t n_tokens, const int32_t* rest, int64_t n_rest, const void* background, int64_t ldb,
+                 void* out, int64_t ldo, int64_t rows, int64_t C, int dtype, void* stream);
+
 /* Linear forward for callers that cannot allocate device memory (no counterpart in the reference, which
  * allocates its intermediates with torch.empty on every call):
  *   out = fused_gemm(quant_rows(x), w, s_col, bias)      -- Int8Linear without a low-rank branch.

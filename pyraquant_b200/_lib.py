@@ -75,6 +75,8 @@ SIGNATURES = {
                                    c_int64, c_int64, c_int64, c_int64, c_void_p, c_size_t, c_void_p]),
     "pq_scatter_rows": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int64,
                                 c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p]),
+    "pq_fuse_rows": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p, c_int64,
+                             c_void_p, c_int64, c_void_p, c_int64, c_int64, c_int64, c_int, c_void_p]),
     "pq_noalloc_scratch_bytes": (c_size_t, []),
     "pq_int8_linear_noalloc": (c_int, [c_void_p, c_int, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
                                        c_int64, c_int64, c_int64, c_int64, POINTER(c_void_p), c_void_p]),

@@ -161,13 +161,39 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads, 4)
 pq_scatter_rows_kernel(const T* __restrict__ y, int64_t ldy, int64_t M_act, const int32_t* __restrict__ tokens,
                        const int32_t* __restrict__ ptr, const int32_t* __restrict__ src,
-                       const float* __restrict__ beta, int64_t n_tokens, T* __restrict__ canvas, int64_t ldc,
-                       int64_t rows, int nchunk) {
+                       const float* __restrict__ beta, int64_t n_tokens, const T* bg, int64_t ldb, T* canvas, int64_t ldc,
+                       int64_t rows, int nchunk, const int32_t* __restrict__ rest, int64_t n_rest, int scatter_blocks) {
   __shared__ BlendToken blend_list[kTokPerBlock];
   __shared__ int2 copy_list[kTokPerBlock];          // (canvas token, routed row)
   __shared__ int n_blend, n_copy;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
+  if (static_cast<int>(blockIdx.x) >= scatter_blocks) {
+    // out-of-place form: the rows no patch touches go over unchanged, in blocks of their own.  HBM-bound; each row moves
+    // once, where a copy of the whole background before the scatter moved the touched rows twice (256 x 256 canvas of 3072
+    // channels, a third touched: 833 instead of 1100 MB, the routed MLP that ends in it 1965 -> 1940 us).
+    const int64_t i0 = static_cast<int64_t>(static_cast<int>(blockIdx.x) - scatter_blocks) * kTokPerBlock;
+    for (int64_t i = i0 + warp; i < i0 + kTokPerBlock && i < n_rest; i += kWarps) {
+      const int64_t r = rest[i];
+      if (r < 0 || r >= rows) continue;
+      const uint4* b0 = reinterpret_cast<const uint4*>(bg + r * ldb);
+      uint4* o0 = reinterpret_cast<uint4*>(canvas + r * ldc);
+      for (int base = 0; base < nchunk; base += 32 * kCopyBatch) {
+        uint4 v[kCopyBatch];
+#pragma unroll
+        for (int j = 0; j < kCopyBatch; ++j) {
+          const int c = base + j * 32 + lane;
+          if (c < nchunk) v[j] = ld_stream_v4(b0 + c);
+        }
+#pragma unroll
+        for (int j = 0; j < kCopyBatch; ++j) {
+          const int c = base + j * 32 + lane;
+          if (c < nchunk) st_v4(o0 + c, v[j]);
+        }
+      }
+    }
+    return;
+  }
   if (threadIdx.x == 0) { n_blend = 0; n_copy = 0; }
   __syncthreads();
   const int64_t tk = static_cast<int64_t>(blockIdx.x) * kTokPerBlock + threadIdx.x;
@@ -222,6 +248,7 @@ pq_scatter_rows_kernel(const T* __restrict__ y, int64_t ldy, int64_t M_act, cons
     tb.setup(bt.b0, bt.b1, bt.bsum);
     const bool need_bg = tb.need_bg;
     uint4* crow = reinterpret_cast<uint4*>(canvas + static_cast<int64_t>(bt.tok) * ldc);
+    const uint4* brow = reinterpret_cast<const uint4*>(bg + static_cast<int64_t>(bt.tok) * ldb);   // == crow in place
     if (bt.nv <= 2) {
       const uint4* y0 = reinterpret_cast<const uint4*>(y + static_cast<int64_t>(bt.r0) * ldy);
       const uint4* y1 = reinterpret_cast<const uint4*>(y + static_cast<int64_t>(bt.r1) * ldy);
@@ -233,7 +260,7 @@ pq_scatter_rows_kernel(const T* __restrict__ y, int64_t ldy, int64_t M_act, cons
         if (c < nchunk) {
           if (bt.nv >= 1) v0[j] = ld_stream_v4(y0 + c);
           if (bt.nv >= 2) v1[j] = ld_stream_v4(y1 + c);
-          if (need_bg) bgv[j] = ld_v4(crow + c);
+          if (need_bg) bgv[j] = ld_v4(brow + c);
         }
       }
       if (tb.packed) {
@@ -268,7 +295,7 @@ pq_scatter_rows_kernel(const T* __restrict__ y, int64_t ldy, int64_t M_act, cons
           if (r < 0 || r >= M_act) continue;
           tb.add(local, ld_stream_v4(reinterpret_cast<const uint4*>(y + r * ldy) + c), b);
         }
-        tb.finish(local, need_bg ? ld_v4(crow + c) : zero4, crow + c);
+        tb.finish(local, need_bg ? ld_v4(brow + c) : zero4, crow + c);
       }
     }
   }
@@ -276,11 +303,14 @@ pq_scatter_rows_kernel(const T* __restrict__ y, int64_t ldy, int64_t M_act, cons
 
 template <typename T>
 int launch_scatter(const void* y, int64_t ldy, int64_t M_act, const int32_t* tokens, const int32_t* ptr, const int32_t* src,
-                   const float* beta, int64_t n_tokens, void* canvas, int64_t ldc, int64_t rows, int nchunk, cudaStream_t st) {
+                   const float* beta, int64_t n_tokens, const void* bg, int64_t ldb, void* canvas, int64_t ldc, int64_t rows,
+                   int nchunk, const int32_t* rest, int64_t n_rest, cudaStream_t st) {
   const int64_t blocks = (n_tokens + kTokPerBlock - 1) / kTokPerBlock;
-  if (blocks > 0x7fffffffLL) return PQ_ERR_SHAPE;
-  pq_scatter_rows_kernel<T><<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(
-      static_cast<const T*>(y), ldy, M_act, tokens, ptr, src, beta, n_tokens, static_cast<T*>(canvas), ldc, rows, nchunk);
+  const int64_t rest_blocks = (n_rest + kTokPerBlock - 1) / kTokPerBlock;
+  if (blocks + rest_blocks > 0x7fffffffLL) return PQ_ERR_SHAPE;
+  pq_scatter_rows_kernel<T><<<static_cast<unsigned>(blocks + rest_blocks), kThreads, 0, st>>>(
+      static_cast<const T*>(y), ldy, M_act, tokens, ptr, src, beta, n_tokens, static_cast<const T*>(bg), ldb,
+      static_cast<T*>(canvas), ldc, rows, nchunk, rest, n_rest, static_cast<int>(blocks));
   PQ_CUDA_TRY(cudaGetLastError());
   return PQ_OK;
 }
@@ -302,7 +332,31 @@ extern "C" int pq_scatter_rows(const void* y, int64_t ldy, int64_t M_act, const 
   const int nchunk = static_cast<int>(C >> 3);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (dtype == PQ_DTYPE_BF16)
-    return launch_scatter<__nv_bfloat16>(y, ldy, M_act, tokens, ptr, src, beta, n_tokens, canvas, ldc, rows, nchunk, st);
-  return launch_scatter<__half>(y, ldy, M_act, tokens, ptr, src, beta, n_tokens, canvas, ldc, rows, nchunk, st);
+    return launch_scatter<__nv_bfloat16>(y, ldy, M_act, tokens, ptr, src, beta, n_tokens, canvas, ldc, canvas, ldc, rows, nchunk,
+                                         nullptr, 0, st);
+  return launch_scatter<__half>(y, ldy, M_act, tokens, ptr, src, beta, n_tokens, canvas, ldc, canvas, ldc, rows, nchunk, nullptr,
+                                0, st);
 }
 
+extern "C" int pq_fuse_rows(const void* y, int64_t ldy, int64_t M_act, const int32_t* tokens, const int32_t* ptr,
+                            const int32_t* src, const float* beta, int64_t n_tokens, const int32_t* rest, int64_t n_rest,
+                            const void* background, int64_t ldb, void* out, int64_t ldo, int64_t rows, int64_t C, int dtype,
+                            void* stream) {
+  if (M_act < 0 || n_tokens < 0 || n_rest < 0 || rows < 0 || C <= 0 || C > 0x7fffffffLL || ldy < C || ldb < C || ldo < C)
+    return PQ_ERR_SHAPE;
+  if (dtype != PQ_DTYPE_BF16 && dtype != PQ_DTYPE_FP16) return PQ_ERR_DTYPE;
+  if (n_tokens + n_rest == 0) return PQ_OK;
+  if (background == nullptr || out == nullptr || (n_rest > 0 && rest == nullptr) ||
+      (n_tokens > 0 && (y == nullptr || tokens == nullptr || ptr == nullptr || src == nullptr || beta == nullptr)))
+    return PQ_ERR_NULL;
+  if (C % 8 != 0 || ldy % 8 != 0 || ldb % 8 != 0 || ldo % 8 != 0 || !aligned_to(y, 16) || !aligned_to(background, 16) ||
+      !aligned_to(out, 16))
+    return PQ_ERR_ALIGN;
+  const int nchunk = static_cast<int>(C >> 3);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (dtype == PQ_DTYPE_BF16)
+    return launch_scatter<__nv_bfloat16>(y, ldy, M_act, tokens, ptr, src, beta, n_tokens, background, ldb, out, ldo, rows, nchunk,
+                                         rest, n_rest, st);
+  return launch_scatter<__half>(y, ldy, M_act, tokens, ptr, src, beta, n_tokens, background, ldb, out, ldo, rows, nchunk, rest,
+                                n_rest, st);
+}

@@ -572,6 +572,26 @@ def _scatter_rows_impl(y: Tensor, tokens: Tensor, ptr: Tensor, src: Tensor, beta
     _lib.check(rc, "pq_scatter_rows")
 
 
+def fuse_rows(background: Tensor, y: Tensor, tokens: Tensor, ptr: Tensor, src: Tensor, beta: Tensor, rest: Tensor) -> Tensor:
+    """A new [rows, C] tensor: the routed rows blended over `background` at `tokens`, the background's rows at `rest`
+    (pq_fuse_rows)."""
+    assert y.is_cuda and background.is_cuda and y.dtype == background.dtype and y.dim() == 2 and background.dim() == 2
+    assert y.stride(1) == 1 and background.stride(1) == 1 and y.shape[1] == background.shape[1]
+    for v in (tokens, ptr, src, rest):
+        assert v.is_cuda and v.dtype == torch.int32 and v.is_contiguous()
+    assert beta.is_cuda and beta.dtype == torch.float32 and beta.is_contiguous()
+    rows, C = background.shape
+    check_scatter_extents(y.shape[0], rows, tokens, ptr, src, beta)
+    assert tokens.numel() + rest.numel() == rows, (tokens.numel(), rest.numel(), rows)
+    out = torch.empty((rows, C), dtype=y.dtype, device=background.device)
+    with _on_device(background):
+        rc = _LIB().pq_fuse_rows(y.data_ptr(), max(y.stride(0), C), y.shape[0], tokens.data_ptr(), ptr.data_ptr(), src.data_ptr(),
+                                 beta.data_ptr(), tokens.numel(), rest.data_ptr(), rest.numel(), background.data_ptr(),
+                                 max(background.stride(0), C), out.data_ptr(), C, rows, C, _dt(y.dtype), _stream(background))
+    _lib.check(rc, "pq_fuse_rows")
+    return out
+
+
 # ------------------------------------------------------------------------------------------------ custom ops
 # torch.library schemas cannot carry torch.dtype arguments portably, so out_dtype travels as the dtype code.
 _CODE2DT = {_lib.DTYPE_BF16: torch.bfloat16, _lib.DTYPE_FP16: torch.float16}

@@ -141,15 +141,22 @@ class RoutePlan:
     def n_rows(self) -> int:
         return int(self.row_idx.shape[0])
 
+    def untouched(self) -> np.ndarray:
+        """int32: the canvas tokens without a contributor, ascending."""
+        mask = np.ones(int(self.token_hw[0]) * int(self.token_hw[1]), dtype=bool)
+        mask[self.tokens] = False
+        return np.flatnonzero(mask).astype(np.int32)
+
     def to(self, device) -> Dict[str, torch.Tensor]:
         key = str(torch.device(device))
-        if key not in self.device_cache:
+        if "rest" not in self.device_cache.get(key, ()):
             self.device_cache[key] = {
                 "row_idx": torch.from_numpy(self.row_idx).to(device),
                 "tokens": torch.from_numpy(self.tokens).to(device),
                 "ptr": torch.from_numpy(self.ptr).to(device),
                 "src": torch.from_numpy(self.src).to(device),
                 "beta": torch.from_numpy(self.beta).to(device),
+                "rest": torch.from_numpy(self.untouched()).to(device),
             }
         return self.device_cache[key]
 
@@ -294,6 +301,13 @@ def fuse_rows(background: torch.Tensor, y: torch.Tensor, plan: RoutePlan) -> tor
     b, H, W, C = background.shape
     if int(b) != 1:
         raise ValueError("Only batch-one full-image fusion is supported")
-    out = background.reshape(H * W, C).clone()
+    bg = background.reshape(H * W, C)
+    if (_eager() and bg.is_cuda and y.device == bg.device and y.dtype == bg.dtype and y.dtype in ops._DT and C % 8 == 0
+            and bg.stride(1) == 1 and bg.stride(0) % 8 == 0 and bg.data_ptr() % 16 == 0 and y.dim() == 2 and y.stride(1) == 1
+            and y.stride(0) % 8 == 0 and y.data_ptr() % 16 == 0 and (H, W) == tuple(plan.token_hw)):
+        d = plan.to(bg.device)
+        if d["tokens"].numel() + d["rest"].numel() == H * W:          # a hand-made plan may list a token twice
+            return ops.fuse_rows(bg, y, d["tokens"], d["ptr"], d["src"], d["beta"], d["rest"]).reshape(1, H, W, C)
+    out = bg.clone()
     scatter_rows_(y, plan, out)
     return out.reshape(1, H, W, C)

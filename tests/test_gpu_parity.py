@@ -1254,3 +1254,28 @@ def test_linear_in_one_call(cuda_dev, M, K, N, lowrank, dtype):
         bare.lr_B = (torch.randn(32, N, generator=g) * 0.05).to(dtype).to(cuda_dev)
         assert torch.equal(bare(x), int8_exec.int8_gemm_lr(xq, sx, bare.weight_int8, bare.w_scale, bare.bias, bare._down(x),
                                                            bare.lr_B, dtype))
+
+
+# ------------------------------------------------------------------------------------------------ out-of-place fusion
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("hw,C,halo,boxes", [((32, 32), 64, 2, [(0, 16, 0, 32), (16, 32, 16, 48), (48, 64, 0, 16)]),
+                                             ((17, 9), 8, 1, [(0, 2, 0, 2)]), ((8, 8), 3072, 0, [(0, 16, 0, 16)]),
+                                             ((24, 40), 264, 3, [(40, 48, 72, 80), (0, 8, 0, 8)])])
+def test_fuse_rows_out_of_place(cuda_dev, dtype, hw, C, halo, boxes):
+    """`fuse_rows` in one launch == the in-place scatter on a clone, bit for bit, on contiguous and row-strided backgrounds:
+    untouched rows (signed zeros included) go over as they are, the background itself is left alone; whole canvas covered,
+    a single patch, patches at both ends of the token list."""
+    g = torch.Generator().manual_seed(C + halo)
+    H, W = hw
+    plan = routing.build_route_plan(hw, boxes, halo, dtype=dtype)
+    wide = torch.randn(1, H, W, C + 8, generator=g).to(dtype)
+    wide[0, H - 1, W - 1] = -0.0
+    y = torch.randn(plan.n_rows, C, generator=g).to(dtype).to(cuda_dev)
+    for bg in (wide[..., :C].contiguous().to(cuda_dev), wide.to(cuda_dev)[..., :C]):
+        before = bg.clone()
+        want = bg.reshape(H * W, C).clone().contiguous()
+        routing.scatter_rows_(y, plan, want)
+        got = routing.fuse_rows(bg, y, plan)
+        assert got.shape == (1, H, W, C)
+        assert torch.equal(got.reshape(H * W, C).view(torch.int16), want.view(torch.int16))
+        assert torch.equal(bg, before)
