@@ -1256,6 +1256,51 @@ def test_linear_in_one_call(cuda_dev, M, K, N, lowrank, dtype):
                                                            bare.lr_B, dtype))
 
 
+class _Doubled(nn.Module):
+    def forward(self, t):
+        return t * 2
+
+    def right_inverse(self, t):
+        return t / 2
+
+
+@pytest.mark.parametrize("where", ["parameter", "parametrised", "buffer"])
+@pytest.mark.parametrize("names", [("bias",), ("lr_A", "lr_B"), ("w_scale",), ("weight_int8",), ("bias", "lr_A", "lr_B", "w_scale")])
+def test_linear_operands_wherever_the_module_keeps_them(cuda_dev, names, where):
+    """A layer's tensors take part in `forward` as `self.<name>` gives them, also after they became Parameters (an assignment
+    or `load_state_dict(assign=True)`) or were parametrised: bit-equal to the separate operators and to `forward_into`, which
+    reads the attributes."""
+    g = torch.Generator().manual_seed(len(names))
+    M, K, N, dtype = 70, 512, 264, torch.bfloat16
+    m = _toy_layer(cuda_dev, g, K, N, lowrank="lr_A" in names, bias="bias" not in names, dtype=dtype)
+    x = rand_act(M, K, dtype, 3).to(cuda_dev)
+    before = m(x)
+    for n in names:
+        t = torch.randn(N, generator=g).to(cuda_dev) if n == "bias" else getattr(m, n).clone()
+        if where == "buffer":
+            if n == "bias":
+                del m.bias
+                m.register_buffer("bias", t)
+            else:
+                setattr(m, n, t)
+        elif where == "parameter" or not t.is_floating_point():
+            setattr(m, n, nn.Parameter(t, requires_grad=t.is_floating_point()))
+        else:
+            if n == "bias":
+                m.bias = nn.Parameter(t)
+            from torch.nn.utils import parametrize
+            parametrize.register_parametrization(m, n, _Doubled(), unsafe=True)
+    y = m(x)
+    xq, sx = int8_exec.quant_rows(x)
+    if m.lr_A is not None:
+        want = int8_exec.int8_gemm_lr(xq, sx, m.weight_int8, m.w_scale, m.bias, m._down(x), m.lr_B, dtype)
+    else:
+        want = int8_exec.int8_gemm_fused(xq, sx, m.weight_int8, m.w_scale, m.bias, dtype)
+    assert torch.equal(y, want)
+    assert torch.equal(m.forward_into(x, torch.empty_like(y)), want)
+    assert ("bias" in names) == (not torch.equal(y, before))
+
+
 # ------------------------------------------------------------------------------------------------ out-of-place fusion
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("hw,C,halo,boxes", [((32, 32), 64, 2, [(0, 16, 0, 32), (16, 32, 16, 48), (48, 64, 0, 16)]),
