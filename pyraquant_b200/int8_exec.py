@@ -372,6 +372,10 @@ class Int8Linear(nn.Module):
                 return None
             rank = 32
             lr_b, lbt, at = self.lr_B, self._lr_Bt(), self._lr_At()
+            # the library sees bare pointers: factors that do not fit the layer must not get there
+            assert at.shape == (32, K) and at.device == x2.device, (tuple(at.shape), at.device)
+            if lr_b.stride(1) != 1:
+                return None
             low = (lr_b.data_ptr(), lbt.data_ptr(), at.data_ptr())
         else:
             low = None
@@ -382,9 +386,13 @@ class Int8Linear(nn.Module):
         c = self.__dict__.get("_lean_cache")
         if c is None or c[0] != key:
             N = self.out_features
-            assert sc.dtype == torch.float32 and (bias is None or bias.dtype == torch.float32), "w_scale and bias are fp32 buffers"
-            assert sc.numel() == N and (bias is None or bias.numel() == N)
-            assert w.dtype == torch.int8 and w.stride(1) == 1 and K == w.shape[1], (w.shape, K)
+            assert w.dtype == torch.int8 and w.stride(1) == 1 and w.shape == (N, K), (w.shape, K)
+            for v in (sc, bias):
+                assert v is None or (v.dtype == torch.float32 and v.numel() == N and v.device == x2.device), \
+                    "w_scale and bias are fp32 buffers of the layer's device, one entry per output channel"
+                if v is not None and not v.is_contiguous():
+                    return None
+            assert low is None or (lr_b.shape == (32, N) and lr_b.device == x2.device), (tuple(lr_b.shape), lr_b.device)
             ws = ops.status_word(x2.device)
             d = ops._lib.LinearDesc(w=w.data_ptr(), s_col=sc.data_ptr(), bias=bias.data_ptr() if bias is not None else None,
                                     lb=low[0] if low else None, lb_t=low[1] if low else None, a_t=low[2] if low else None,

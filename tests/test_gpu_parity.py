@@ -1301,6 +1301,31 @@ def test_linear_operands_wherever_the_module_keeps_them(cuda_dev, names, where):
     assert ("bias" in names) == (not torch.equal(y, before))
 
 
+def test_linear_refuses_operands_that_do_not_fit(cuda_dev):
+    """The library gets bare pointers, so a factor, scale or bias of another extent or device is an AssertionError before
+    anything is launched; a strided bias is read through its strides."""
+    g = torch.Generator().manual_seed(9)
+    M, K, N, dtype = 70, 576, 264, torch.bfloat16
+    x = rand_act(M, K, dtype, 4).to(cuda_dev)
+    rnd = lambda *s: (torch.randn(*s, generator=g) * 0.05).to(dtype).to(cuda_dev)
+    bad = [("lr_A", rnd(K - 64, 32)), ("lr_A", rnd(K + 64, 32)), ("lr_A", rnd(K, 32).cpu()), ("lr_B", rnd(32, N - 8)),
+           ("lr_B", rnd(32, N).cpu()), ("w_scale", torch.rand(N - 8, device=cuda_dev)), ("w_scale", torch.rand(N)),
+           ("bias", torch.rand(N + 8, device=cuda_dev)), ("bias", torch.rand(N)),
+           ("weight_int8", torch.zeros(N - 8, K, dtype=torch.int8, device=cuda_dev))]
+    for warm in (False, True):
+        for name, t in bad:
+            m = _toy_layer(cuda_dev, g, K, N, lowrank=True, dtype=dtype)
+            if warm:
+                m(x)
+            setattr(m, name, t)
+            with pytest.raises(AssertionError):
+                m(x)
+    m = _toy_layer(cuda_dev, g, K, N, lowrank=True, dtype=dtype)
+    want = m(x)
+    m.bias = torch.stack([m.bias, m.bias + 1], dim=1)[:, 0]
+    assert not m.bias.is_contiguous() and torch.equal(m(x), want)
+
+
 # ------------------------------------------------------------------------------------------------ out-of-place fusion
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("hw,C,halo,boxes", [((32, 32), 64, 2, [(0, 16, 0, 32), (16, 32, 16, 48), (48, 64, 0, 16)]),
