@@ -36,24 +36,24 @@ constexpr int pair_threads(int ew) { return (3 + ew) * 32; }
 constexpr int kShortK = 2048;              // up to this K the sixteen-warp epilogue is used,
 constexpr int kFewBlocks = 160;            // and up to this many k-blocks per pair
 
-// WIDE: the sixteen-warp epilogue without low-rank term, whose output tiles leave through shared memory: one operand stage
-// less (short K needs few), two 2 KB staging blocks per epilogue warp where the t / lbT tiles of the other form are.
-template <bool WIDE>
+// The sixteen-warp epilogue without low-rank term stages its output tiles where the t / lbT tiles of the other form are, a
+// 2 KB block per warp.  Two blocks per warp would cost an operand stage, which is worth more: 16384 x 1280 -> 1280 31.2 us
+// with five stages and two blocks, 27.4 us with six and one.
 struct PairSmem {
-  static constexpr int kStages = WIDE ? PSTAGES - 1 : PSTAGES;
   static constexpr int kABytes = BM * BK;
   static constexpr int kBBytes = kHalfB * BK;
   static constexpr int kStageBytes = kABytes + kBBytes;            // per CTA
-  static constexpr int kTOff = kStages * kStageBytes;
+  static constexpr int kTOff = PSTAGES * kStageBytes;
   static constexpr int kTBytes = BM * kRowBytesLr;                 // per CTA: its 128 rows of t
   static constexpr int kLbOff = kTOff + 2 * kTBytes;
   static constexpr int kLbBytes = kHalfB * kRowBytesLr;            // per CTA: its 128 rows of lbT
   static constexpr int kStageBlock = 16 * 64 * 2;                  // 16 rows x 64 columns of output
-  static constexpr int kScolOff = WIDE ? kTOff + 16 * 2 * kStageBlock : kLbOff + 2 * kLbBytes;   // two lbT buffers: consecutive column tiles alternate
+  static_assert(16 * kStageBlock <= 2 * (kTBytes + kLbBytes), "staging blocks of sixteen warps");
+  static constexpr int kScolOff = kLbOff + 2 * kLbBytes;            // two lbT buffers: consecutive column tiles alternate
   static constexpr int kBiasOff = kScolOff + PBN * 4;
   static constexpr int kBarOff = kBiasOff + PBN * 4;
   // full[S], empty[S], tfull[2], tempty[2], t_full[2], lb_full[2], ylr_ready[2][chunks], lr_done[2][chunks]
-  static constexpr int kNumBars = 2 * kStages + 8 + 4 * kLrChunks;
+  static constexpr int kNumBars = 2 * PSTAGES + 8 + 4 * kLrChunks;
   static constexpr int kMiscOff = kBarOff + kNumBars * 8;
   static constexpr int kTotal = kMiscOff + 16 + 64;      // + time stamps of the cycle-counter experiments
   static_assert(kTotal <= 232448, "exceeds the 227 KB shared memory of one CTA");
@@ -254,14 +254,13 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
                                const __grid_constant__ CUtensorMap tmW1, const __grid_constant__ CUtensorMap tmT, const __grid_constant__ CUtensorMap tmLbT,
                                const __grid_constant__ CUtensorMap tmOut, const GemmParams p) {
   constexpr bool WIDE = EW == 16 && !HAS_LR;
-  using L = PairSmem<WIDE>;
-  constexpr int kStages = L::kStages;
+  using L = PairSmem;
   static_assert(EW == 8 || EW == 16, "eight or sixteen epilogue warps");
   constexpr int kLrWarp = 2 + EW;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L::kBarOff);
-  uint64_t* empty_bar = full_bar + kStages;
-  uint64_t* tfull_bar = empty_bar + kStages;
+  uint64_t* empty_bar = full_bar + PSTAGES;
+  uint64_t* tfull_bar = empty_bar + PSTAGES;
   uint64_t* tempty_bar = tfull_bar + 2;
   uint64_t* t_full = tempty_bar + 2;
   uint64_t* lb_full = t_full + 2;
@@ -290,7 +289,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmW1);
     if (HAS_LR) { tma_prefetch_desc(&tmT); tma_prefetch_desc(&tmLbT); }
-    for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int s = 0; s < PSTAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull_bar[b], 1); mbar_init(&tempty_bar[b], 2 * EW);
       mbar_init(&t_full[b], 1);
@@ -363,7 +362,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
           if (p.l2_hints & 1) tma_load_2d_pair_hint(a_s + L::kABytes, wm, fb, kb * BK, nhalf0, pol_w);
           else tma_load_2d_pair(a_s + L::kABytes, wm, fb, kb * BK, nhalf0);
           ++issued;
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+          if (++stage == PSTAGES) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
         if (HAS_LR) {
@@ -377,9 +376,9 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
       }
       // copies in flight must land before the CTA may exit: the last stages issued are consumed by MMAs whose
       // completion is committed to this CTA's empty barriers
-      const int pending = issued < kStages ? static_cast<int>(issued) : kStages;
+      const int pending = issued < PSTAGES ? static_cast<int>(issued) : PSTAGES;
       for (int i = 0; i < pending; ++i) {
-        if (--stage < 0) { stage = kStages - 1; phase ^= 1u; }
+        if (--stage < 0) { stage = PSTAGES - 1; phase ^= 1u; }
         if (!wait_or_abort(&empty_bar[stage], phase, abort_flag)) {
           for (int k = 0; k < 64; ++k) __nanosleep(1000);
           break;
@@ -425,7 +424,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
             tc_mma_i8_pair(d_tmem, a_desc + static_cast<uint64_t>(2 * k), b_desc + static_cast<uint64_t>(2 * k), idesc,
                            (kb > 0 || k > 0) ? 1u : 0u);
           commit_both(&empty_bar[stage]);
-          if (++stage == kStages) { stage = 0; phase ^= 1u; }
+          if (++stage == PSTAGES) { stage = 0; phase ^= 1u; }
         }
         if (!ok) break;
         commit_both(&tfull_bar[buf]);
@@ -478,8 +477,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
     const int quarter = warp & 3;
     const int half = ((warp - 2) >> 2) & 1;
     // Sixteen warps with a low-rank term: warps 2..9 take the first 16 rows of each 32-row lane quarter, warps 10..17 the
-    // other 16, of every chunk.  Without one (WIDE) a warp takes all 32 rows of 64 columns, so that the column scales and
-    // the bias of its columns are read from shared memory once per tile.
+    // other 16, of every chunk.  Without one (WIDE) a warp takes all 32 rows of 64 columns.
     constexpr int MBN = EW == 16 && !WIDE ? 1 : 2;       // 16-row blocks per warp
     const int mb_base = EW == 16 && !WIDE ? ((warp - 2) >> 3) : 0;
     const int colg = (warp - 2) >> 2;                    // WIDE: columns [64 colg, +64) of the tile
@@ -684,61 +682,63 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
         }
       };
 
-      // WIDE tiles of a plain call go out through shared memory: a warp's rounded 32 x 64 block in the 128-byte-swizzled
+      // WIDE tiles of a plain call go out through shared memory: a warp's rounded 16 x 64 block in the 128-byte-swizzled
       // layout, one TMA store each (TMA clips at M and N).  No in-quad transposes, row predicates or flag tests per store,
-      // the hardware conversion instead of five instructions, the column data read once per tile, and the accumulator
-      // handed back as soon as it is in registers.  65536 x 640 -> 5120 fp16 264 -> 237 us, 671 MB of output that a plain
-      // fill takes 173 us for; 8.6 instead of 14.2 warp instructions per element.  What is left is the store path: the
-      // same time with two groups of eight warps alternating tiles, and 271 us with one thread issuing all stores.
+      // the hardware conversion instead of five instructions, and the accumulator handed back as soon as it is in registers.
+      // A block is written over the previous one only when its words are ready, so that the store before it has the time of
+      // the arithmetic to read it.  bf16, us, against the same warps with register stores: 65536 x 640 -> 5120 285 -> 212
+      // (671 MB of output that a plain fill takes 173 us for), 16384 x 1280 -> 10240 179 -> 162, 16896 x 1536 -> 6144
+      // 118 -> 113.  Waiting for the previous store before the arithmetic: 65536 x 640 -> 640 with the GELU 47.7 instead of
+      // 44.6 us.  The same time with two groups of eight warps alternating tiles; slower with one thread issuing all stores.
       auto staged_tile = [&](auto act) {                     // act: with the GELU (two copies, so that neither carries the other's code)
-        uint32_t v0[16], v1[16];
-        uint8_t* const blk = smem + L::kTOff + (warp - 2) * 2 * L::kStageBlock;     // rows 0-15, then rows 16-31
+        uint32_t v0[16], v1[16], words[2][8];
+        uint8_t* const blk = smem + L::kTOff + (warp - 2) * L::kStageBlock;
         uint8_t* const mine = blk + g * 128 + q * 4;
         tmem_ld_16x256b_x4(unit_addr(0, 0), v0);
-        if (lane == 0) bulk_wait_group_read0();              // the previous tile's stores have read the two blocks
-        __syncwarp();
 #pragma unroll
-        for (int hc = 0; hc < 2; ++hc) {                     // 32 columns, both 16-row blocks
-          float2 sc[4], bi[4];
+        for (int mb = 0; mb < 2; ++mb) {                     // 16 rows
+          const float2 srA = make_float2(srow[mb][0], srow[mb][0]), srB = make_float2(srow[mb][1], srow[mb][1]);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            sc[j] = *reinterpret_cast<const float2*>(scol_s + colg * UNIT_N + (hc * 4 + j) * 8 + 2 * q);
-            bi[j] = *reinterpret_cast<const float2*>(bias_s + colg * UNIT_N + (hc * 4 + j) * 8 + 2 * q);
-          }
-#pragma unroll
-          for (int mb = 0; mb < 2; ++mb) {
-            uint32_t (&v)[16] = mb == 0 ? v0 : v1;
+          for (int hc = 0; hc < 2; ++hc) {                   // 32 columns
+            uint32_t (&v)[16] = hc == 0 ? v0 : v1;
             tc_wait_ld();
-            if (mb == 0) tmem_ld_16x256b_x4(unit_addr(0, 1) + hc * 32, v1);
-            else if (hc == 0) tmem_ld_16x256b_x4(unit_addr(0, 0) + 32, v0);
+            if (hc == 0) tmem_ld_16x256b_x4(unit_addr(0, mb) + 32, v1);
+            else if (mb == 0) tmem_ld_16x256b_x4(unit_addr(0, 1), v0);
             if (mb == 1 && hc == 1) {                        // everything is in registers: the accumulator is free
               tc_fence_before();
               __syncwarp();
               if (lane == 0) mbar_arrive_cluster(leader_addr(&tempty_bar[buf]));
             }
-            const float2 srA = make_float2(srow[mb][0], srow[mb][0]), srB = make_float2(srow[mb][1], srow[mb][1]);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
+              const int cl = colg * UNIT_N + (hc * 4 + j) * 8 + 2 * q;
+              const float2 sc = *reinterpret_cast<const float2*>(scol_s + cl), bi = *reinterpret_cast<const float2*>(bias_s + cl);
               const float2 pA = make_float2(__int2float_rn(static_cast<int32_t>(v[4 * j + 0])), __int2float_rn(static_cast<int32_t>(v[4 * j + 1])));
               const float2 pB = make_float2(__int2float_rn(static_cast<int32_t>(v[4 * j + 2])), __int2float_rn(static_cast<int32_t>(v[4 * j + 3])));
-              const float2 yA = __fmul2_rn(pA, __fmul2_rn(srA, sc[j])), yB = __fmul2_rn(pB, __fmul2_rn(srB, sc[j]));
+              const float2 yA = __fmul2_rn(pA, __fmul2_rn(srA, sc)), yB = __fmul2_rn(pB, __fmul2_rn(srB, sc));
               // scalar additions: packed ones, even written as add.rn.f32x2, get contracted with the products
-              uint32_t wA = pack2(__fadd_rn(yA.x, bi[j].x), __fadd_rn(yA.y, bi[j].y), OutT{});
-              uint32_t wB = pack2(__fadd_rn(yB.x, bi[j].x), __fadd_rn(yB.y, bi[j].y), OutT{});
+              uint32_t wA = pack2(__fadd_rn(yA.x, bi.x), __fadd_rn(yA.y, bi.y), OutT{});
+              uint32_t wB = pack2(__fadd_rn(yB.x, bi.x), __fadd_rn(yB.y, bi.y), OutT{});
               if constexpr (decltype(act)::value) { wA = gelu_word<OutT>(wA); wB = gelu_word<OutT>(wB); }
-              // 16-byte column nb of row g sits at nb ^ g (128-byte swizzle): the eight rows of a store hit different banks
-              uint8_t* dst = mine + mb * L::kStageBlock + (((hc * 4 + j) ^ g) << 4);
-              st_shared_u32(dst, wA);
-              st_shared_u32(dst + 8 * 128, wB);              // row g + 8: same swizzle phase
+              words[hc][2 * j] = wA; words[hc][2 * j + 1] = wB;
             }
           }
-        }
-        fence_proxy_async_smem();
-        __syncwarp();
-        const int r_first = row0 + quarter * 32;             // one box of 32 rows: its two blocks are neighbours
-        if (lane == 0 && r_first < row_end && n0 + colg * UNIT_N < p.N) {
-          tma_store_2d(&tmOut, blk, n0 + colg * UNIT_N, r_first);
-          bulk_commit_group();
+          if (lane == 0) bulk_wait_group_read0();            // the previous store of this warp has read the block
+          __syncwarp();
+#pragma unroll
+          for (int nb = 0; nb < 8; ++nb) {
+            // 16-byte column nb of row g sits at nb ^ g (128-byte swizzle): the eight rows of a store hit different banks
+            uint8_t* dst = mine + ((nb ^ g) << 4);
+            st_shared_u32(dst, words[nb >> 2][2 * (nb & 3)]);
+            st_shared_u32(dst + 8 * 128, words[nb >> 2][2 * (nb & 3) + 1]);       // row g + 8: same swizzle phase
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          const int r_first = row0 + quarter * 32 + mb * 16;
+          if (lane == 0 && r_first < row_end && n0 + colg * UNIT_N < p.N) {
+            tma_store_2d(&tmOut, blk, n0 + colg * UNIT_N, r_first);
+            bulk_commit_group();
+          }
         }
       };
 
@@ -849,13 +849,13 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
   }
 }
 
-// Output [M, N] of 16-bit elements, row stride ldo: boxes of 64 columns x 32 rows, 128-byte swizzle (TMA store).
+// Output [M, N] of 16-bit elements, row stride ldo: boxes of 64 columns x 16 rows, 128-byte swizzle (TMA store).
 int make_out_map16(CUtensorMap* map, void* base, int64_t M, int64_t N, int64_t ldo, bool bf16) {
   EncodeTiledFn fn = encode_fn();
   if (fn == nullptr) return PQ_ERR_CUDA;
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(N), static_cast<cuuint64_t>(M)};
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(ldo) * 2};
-  cuuint32_t box[2] = {64, 32};
+  cuuint32_t box[2] = {64, 16};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, base, dims, strides,
                   box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
@@ -886,11 +886,11 @@ int launch_pair_ew(const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtenso
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
   cfg.blockDim = dim3(pair_threads(EW), 1, 1);
-  cfg.dynamicSmemBytes = PairSmem<EW == 16 && !HAS_LR>::kTotal;
+  cfg.dynamicSmemBytes = PairSmem::kTotal;
   cfg.stream = st;
   cfg.attrs = attr; cfg.numAttrs = 1;
   if (max_pairs[dev] == 0) {
-    PQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem<EW == 16 && !HAS_LR>::kTotal));
+    PQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PairSmem::kTotal));
     cfg.gridDim = dim3(2 * sm_count(), 1, 1);
     int n = 0;
     PQ_CUDA_TRY(cudaOccupancyMaxActiveClusters(&n, kern, &cfg));

@@ -311,6 +311,49 @@ def test_gemm_pair_epilogues_bit_equal_on_many_outputs(cuda_dev, dtype, M, N, K,
     assert torch.equal(y, want)
 
 
+def _exact_gemm_operands(cuda_dev, M, N, K, dtype):
+    """Operands whose accumulators are exact in fp64 and below 2^24, and the output of torch's separate fp32 operations."""
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    xq = torch.randint(-127, 128, (M, K), generator=g, device=cuda_dev, dtype=torch.int8)
+    wq = torch.randint(-127, 128, (N, K), generator=g, device=cuda_dev, dtype=torch.int8)
+    sr = torch.rand(M, generator=g, device=cuda_dev) * 0.05 + 0.001
+    sc = torch.rand(N, generator=g, device=cuda_dev) * 2e-4 + 1e-5
+    b = torch.randn(N, generator=g, device=cuda_dev) * 0.01
+    acc = xq.double() @ wq.double().t()
+    assert acc.abs().max().item() < 2 ** 24
+    return xq, wq, sr, sc, b, ((acc.float() * (sr[:, None] * sc[None, :])) + b[None, :]).to(dtype)
+
+
+@pytest.fixture
+def gemm_options():
+    """Sets library options for one test and puts the defaults back."""
+    defaults = {"gemm_pair": 1, "gemm_block_n": 0, "gemm_epi_warps": 0, "gemm_tma_store": 1, "gemm_max_ctas": 0}
+
+    def set_options(**kw):
+        for k, v in {**defaults, **kw}.items():
+            _lib.set_option(k, v)
+    yield set_options
+    set_options()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N,K", [(2049, 1280, 128), (1500, 1032, 1296), (700, 264, 640)])
+def test_gemm_staged_store_over_many_tiles(cuda_dev, gemm_options, dtype, M, N, K):
+    """Sixteen-warp tiles that leave through shared memory, in the kernel users run: two SM pairs go through all tiles, so that
+    staging blocks and accumulators are reused many times; bit-equal to torch's separate operations, and with the GELU to the
+    same tiles stored from registers."""
+    xq, wq, sr, sc, b, want = _exact_gemm_operands(cuda_dev, M, N, K, dtype)
+    gelu = {}
+    for tma in (1, 0):
+        for ctas in (0, 4):
+            gemm_options(gemm_pair=2, gemm_block_n=256, gemm_epi_warps=16, gemm_tma_store=tma, gemm_max_ctas=ctas)
+            assert torch.equal(int8_exec.int8_gemm_fused(xq, sr, wq, sc, b, dtype), want), (tma, ctas)
+            if N % 32 == 0:
+                gelu[tma, ctas] = ops._gemm_impl(xq, sr, wq, sc, b, None, None, dtype, epilogue=ops.EPI_GELU_TANH)
+    assert all(torch.equal(v, next(iter(gelu.values()))) for v in gelu.values())
+    ops.check_device_status(cuda_dev)
+
+
 @pytest.mark.parametrize("pair", [0, 2])
 def test_gemm_accumulators_beyond_24_bits_round_like_the_restatement(cuda_dev, pair):
     """Same-sign codes and K = 8192 give accumulators of 2^24 .. 2^27 with arbitrary low bits: the int32 -> fp32
