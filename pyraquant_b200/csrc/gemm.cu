@@ -516,20 +516,34 @@ int choose_block_n(int64_t M, int64_t N) {
   return 256;
 }
 
-// CTA-pair tiles (256 x 256 on two SMs) or single-CTA ones.  A k-block of a 128 x 128 tile brings in 32 KB for 256 cycles
-// of MMA, one of a pair tile 32 KB per SM for 512: both take the 512 cycles that 32 KB need at the 64 bytes per clock an SM
-// gets from L2, so what counts is the number of tiles an SM goes through, padding included.  Measured (pair / single, us):
-// 3001 x 1808 -> 2376 (2 against 4 tiles) 20.2 / 31, 30000 x 320 -> 320 (4 / 5) 12.8 / 24.6, 65536 x 640 -> 640 (11 / 18)
-// 34.7 / 38.8, 1024 x 12288 -> 3072 rank 32 (1 / 2) 37.4 / 43.8, 700 x 3072 -> 9216 rank 32 (2 / 3) 24.3 / 24.4, and where a
-// short K leaves the longer epilogue of the wide tile exposed 4096 x 640 -> 640 (1 / 2) 8.0 / 7.3.
-bool prefer_pair(int bn, int64_t pair_rows, int64_t M, int64_t N, int64_t K, bool has_lr) {
-  const int64_t pair_tiles = pair_rows * ((N + 255) / 256), pairs = sm_count() / 2;
+// CTA-pair tiles (256 x 256 on two SMs) or single-CTA ones, where 256-column tiles do not fill the SM pairs or waste columns.
+// A k-block of a 128 x 128 tile brings in 32 KB for 256 cycles of MMA, one of a pair tile 32 KB per SM for 512: both take
+// the 512 cycles that 32 KB need at the 64 bytes per clock an SM gets from L2, so what counts is the number of tiles an SM
+// goes through, padding included -- and the epilogue of a tile, which is longer for the pair tile.  `staged`: a plain call whose
+// tiles leave through shared memory (short epilogue); the others store from registers.  us, pair / single, bf16:
+//   N % 128 != 0 (the single kernel's last column tile stores element by element): staged 1024 x 1808 -> 2376 (1 tile / 2)
+//     13.4 / 19.1, 30000 x 320 -> 320 (4 / 5) 15.5 / 25.7, but 30000 x 5120 -> 320 69.1 / 65.0; two tiers 65536 x 640 -> 320
+//     (7 / 11) 45.0 / 50.7; rank 32 65536 x 1808 -> 320 69.1 / 79.4, 3001 x 1808 -> 2376 (2 / 4) 28.6 / 35.7, 30000 x 320 -> 320
+//     37.0 / 30.0;
+//   N % 128 == 0: staged 65536 x 640 -> 640 (11 / 18) 33.2 / 42.0, 3001 x 1808 -> 1920 (2 / 3) 20.1 / 24.9, 4096 x 2560 -> 640
+//     (1 / 2) 13.8 / 13.3, 4096 x 5120 -> 640 20.3 / 23.5; rank 32 65536 x 640 -> 640 76.8 / 58.7, 16384 x 1280 -> 640 (3 / 5)
+//     29.6 / 25.9, 4096 x 1280 -> 1920 (2 / 4) 21.8 / 20.9, 65536 x 1280 -> 1920 (28 / 52) 197 / 242, 65536 x 2560 -> 640 105 / 116, 2048 x 2560 -> 1920 (1 / 2)
+//     18.3 / 17.0, 2048 x 5120 -> 1920 24.9 / 25.9; two tiers 16384 x 640 -> 640 24.3 / 15.4, 8192 x 1280 -> 1920 (4 / 7)
+//     32.2 / 28.1, 4096 x 5120 -> 640 (1 / 2) 23.8 / 23.4, 4096 x 12288 -> 640 39.8 / 46.4.
+bool prefer_pair(int bn, int64_t pair_rows, int64_t M, int64_t N, int64_t K, bool has_lr, bool staged) {
+  int64_t ctas = sm_count();
+  if (options().gemm_max_ctas > 1 && options().gemm_max_ctas < ctas) ctas = options().gemm_max_ctas;
+  const int64_t pair_tiles = pair_rows * ((N + 255) / 256), pairs = ctas / 2;
   if (bn == 256 && pair_tiles >= pairs) return true;
   if (options().gemm_block_n != 0) return false;
   const int64_t pair_steps = (pair_tiles + pairs - 1) / pairs;
-  const int64_t single_steps = (((M + BM - 1) / BM) * ((N + 127) / 128) + sm_count() - 1) / sm_count();
-  if (pair_steps == 1) return single_steps >= 3 || (single_steps == 2 && K >= 2048);
-  return has_lr ? 5 * single_steps >= 8 * pair_steps : single_steps > pair_steps;
+  const int64_t single_steps = (((M + BM - 1) / BM) * ((N + 127) / 128) + ctas - 1) / ctas;
+  const bool fewer = 2 * single_steps >= 3 * pair_steps, far_fewer = 5 * single_steps >= 8 * pair_steps;
+  if (N % 128 != 0)
+    return far_fewer || (staged && single_steps > pair_steps && K <= 2560) || (fewer && (!has_lr || K >= 1280));
+  if (pair_steps == 1) return single_steps >= 2 && K >= (staged || has_lr ? 4096 : 8192);
+  if (staged) return far_fewer || (fewer && K >= 1792);
+  return (far_fewer && K >= 1792) || (has_lr && pair_steps >= 4 && 7 * single_steps >= 12 * pair_steps && K >= 1280);
 }
 
 int gemm_common(const int8_t* xq, int64_t ldx, const float* s_row, const int8_t* w0, const float* sc0,
@@ -584,8 +598,8 @@ int gemm_common(const int8_t* xq, int64_t ldx, const float* s_row, const int8_t*
   p.n_out_more = n_out_more;
   for (int d = 0; d < 7; ++d) p.out_more[d] = d < n_out_more ? out_more[d] : nullptr;
 
-  // CTA-pair kernel: 256-column tiles, enough 256-row tiles to occupy the SM pairs, and the K-major low-rank
-  // factor when there is a low-rank term
+  // CTA-pair kernel: always for the epilogue variants, by size otherwise (prefer_pair); it needs the K-major low-rank factor
+  // when there is a low-rank term
   {
     const int64_t pair_rows = (m_split + 255) / 256 + (M - m_split + 255) / 256;
     const bool pair_legal = (!has_lr || lb_t != nullptr);
@@ -595,7 +609,8 @@ int gemm_common(const int8_t* xq, int64_t ldx, const float* s_row, const int8_t*
       return launch_gemm_pair(out_dtype == PQ_DTYPE_BF16, dbg_acc != nullptr || p.timing != nullptr, xq, ldx, w0, w1, ldw, has_lr ? t : nullptr, ldt,
                               has_lr ? lb_t : nullptr, M, N, K, p, static_cast<cudaStream_t>(stream));
     }
-    const bool want_pair = options().gemm_pair == 2 ? bn == 256 : prefer_pair(bn, pair_rows, M, N, K, has_lr);
+    const bool staged = !has_lr && m_split == M && dbg_acc == nullptr && pair_staged_store(out, ldo);
+    const bool want_pair = options().gemm_pair == 2 || prefer_pair(bn, pair_rows, M, N, K, has_lr, staged);
     if (options().gemm_pair != 0 && pair_legal && want_pair) {
       return launch_gemm_pair(out_dtype == PQ_DTYPE_BF16, dbg_acc != nullptr || p.timing != nullptr, xq, ldx, w0, w1, ldw, has_lr ? t : nullptr, ldt,
                               has_lr ? lb_t : nullptr, M, N, K, p, static_cast<cudaStream_t>(stream));

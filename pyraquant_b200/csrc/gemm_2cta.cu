@@ -870,8 +870,8 @@ int launch_pair_ew(const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtenso
   // sixteen-warp tiles of a plain single-tier call store through shared memory + TMA when the output allows it
   CUtensorMap tmOut = tmA;
   p.tma_store = 0;
-  if (EW == 16 && !HAS_LR && !DBG && p.m_split == p.M && !(p.epi_flags & (PQ_EPI_ACCUMULATE | PQ_EPI_GATE)) && p.n_out_more == 0 && options().gemm_tma_store != 0 &&
-      p.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(p.out) & 15) == 0) {
+  if (EW == 16 && !HAS_LR && !DBG && p.m_split == p.M && !(p.epi_flags & (PQ_EPI_ACCUMULATE | PQ_EPI_GATE)) && p.n_out_more == 0 &&
+      pair_staged_store(p.out, p.ldo)) {
     const int rc = make_out_map16(&tmOut, p.out, p.M, p.N, p.ldo, std::is_same<OutT, __nv_bfloat16>::value);
     if (rc != PQ_OK) return rc;
     p.tma_store = 1;
@@ -948,7 +948,8 @@ template <typename OutT, bool HAS_LR, bool DBG>
 int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtensorMap& tmW1, const CUtensorMap& tmT,
                 const CUtensorMap& tmLbT, GemmParams p, int mt_pairs, int ntl, cudaStream_t st) {
   const int want = options().gemm_epi_warps;
-  const int64_t pairs = sm_count() / 2;
+  int64_t pairs = sm_count() / 2;
+  if (options().gemm_max_ctas > 1 && options().gemm_max_ctas / 2 < pairs) pairs = options().gemm_max_ctas / 2;
   const int64_t kblocks = (static_cast<int64_t>(mt_pairs) * ntl + pairs - 1) / pairs * ((p.K + BK - 1) / BK);
   const bool wide = want == 16 || (want != 8 && (p.K <= kShortK || kblocks <= kFewBlocks));
   if (wide) return launch_pair_ew<OutT, HAS_LR, DBG, 16>(tmA, tmW, tmW1, tmT, tmLbT, p, mt_pairs, ntl, st);

@@ -5,6 +5,12 @@
 
 namespace pq {
 
+// Whether the output rows can leave through shared memory + TMA (sixteen-warp tiles of a plain single-tier call without
+// low-rank term).
+inline bool pair_staged_store(const void* out, int64_t ldo) {
+  return options().gemm_tma_store != 0 && ldo % 8 == 0 && aligned_to(out, 16);
+}
+
 // One or two weight sets (rows [0, p.m_split) use w, the rest w1; w1 is ignored when p.m_split == M).  t / lb_t may both be NULL (no low-rank term); otherwise t [M,32] (row stride ldt) and
 // lb_t [N,32] contiguous in the output dtype.  The tile schedule fields of `p` are filled in here.
 int launch_gemm_pair(bool bf16, bool dbg, const void* xq, int64_t ldx, const void* w, const void* w1, int64_t ldw,

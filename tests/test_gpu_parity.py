@@ -354,6 +354,35 @@ def test_gemm_staged_store_over_many_tiles(cuda_dev, gemm_options, dtype, M, N, 
     ops.check_device_status(cuda_dev)
 
 
+@pytest.mark.parametrize("M,N,K", [(4096, 640, 2560), (4096, 640, 5120), (5000, 640, 640), (9600, 320, 320), (1024, 2376, 1808),
+                                   (700, 3072, 1024), (2048, 264, 96)])
+def test_gemm_kernel_choice_by_size(cuda_dev, gemm_options, M, N, K):
+    """On both sides of the lines between the CTA-pair and the single-CTA kernel: the automatic choice, each kernel forced, and
+    the single-CTA kernel with few CTAs give the same bits, one and two weight tiers, an output with and without room for the
+    staged store; with the rank-32 term they agree to its rounding."""
+    dtype = torch.bfloat16
+    xq, wq, sr, sc, b, want = _exact_gemm_operands(cuda_dev, M, N, K, dtype)
+    mh = M // 2 + 3
+    tiers = torch.cat([want[:mh], (((xq[mh:].double() @ -wq.double().t()).float() * (sr[mh:, None] * (sc * 2)[None, :]))
+                                   + b[None, :]).to(dtype)])
+    g = torch.Generator(device="cuda").manual_seed(N)
+    t = torch.randn(M, 32, generator=g, device=cuda_dev).to(dtype)
+    lb = (torch.randn(32, N, generator=g, device=cuda_dev) * 0.1).to(dtype)
+    lr = []
+    for opt in ({}, {"gemm_pair": 2}, {"gemm_pair": 0}, {"gemm_pair": 0, "gemm_max_ctas": 3}, {"gemm_max_ctas": 6}):
+        gemm_options(**opt)
+        assert torch.equal(int8_exec.int8_gemm_fused(xq, sr, wq, sc, b, dtype), want), opt
+        odd = torch.zeros(M, N + 2, dtype=dtype, device=cuda_dev)[:, :N]            # rows of no 16-byte pitch
+        assert torch.equal(ops._gemm_impl(xq, sr, wq, sc, b, None, None, dtype, out=odd), want), opt
+        assert torch.equal(int8_exec.int8_gemm_grouped(xq, sr, wq, sc, -wq, sc * 2, b, None, None, mh, dtype), tiers), opt
+        lr.append(int8_exec.int8_gemm_lr(xq, sr, wq, sc, b, t, lb, dtype))
+    ref = want.double() + t.double() @ lb.double()
+    for y in lr:
+        # one rounding of the output and one of the intermediate `want`, each at most 2^-9 of its operand
+        assert bool(((y.double() - ref).abs() <= 2.0 ** -8 * (want.double().abs() + ref.abs()) + 1e-6 * (t.double().abs() @ lb.double().abs())).all())
+    ops.check_device_status(cuda_dev)
+
+
 @pytest.mark.parametrize("pair", [0, 2])
 def test_gemm_accumulators_beyond_24_bits_round_like_the_restatement(cuda_dev, pair):
     """Same-sign codes and K = 8192 give accumulators of 2^24 .. 2^27 with arbitrary low bits: the int32 -> fp32
