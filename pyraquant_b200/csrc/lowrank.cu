@@ -6,13 +6,16 @@
 // tcgen05.mma.kind::f16 64 x 32 x 16 (eight per stage) into one of two 32-column accumulators, and four epilogue warps
 // round and store finished tiles while the next tile streams.  A is passed transposed ([32, K], K-contiguous) so
 // that both operands are K-major.  Every wait is bounded (status word, abort flag) like in the GEMM kernels.
+// A single factor is summed in the column slices of the one-launch prologue (quant_down.cu), one accumulator per slice and the
+// slices added in order by the epilogue, so that a row's t is the same bits whichever kernel computes it.
 #include <type_traits>
 
 #include "gemm_common.cuh"
 
 namespace pq {
-// quant_down.cu: t alone, the columns summed in slices over a cluster
-bool lowrank_sliced(int64_t K, int R);
+// quant_down.cu: k-blocks (128 elements) per column slice, and t alone, the columns summed in slices over a cluster
+int lowrank_slice_blocks(int64_t K);
+bool lowrank_few_rows(int64_t M, int64_t K, int R);
 int lowrank_down_sliced(const void* x0, int64_t K0, int64_t ldx0, const void* x1, int64_t K1, int64_t ldx1, int dtype,
                         const void* a_t, int64_t lda, int R, void* t, int64_t ldt, int64_t M, void* workspace, size_t ws_bytes,
                         void* stream);
@@ -33,7 +36,7 @@ struct LowSmem {
   static constexpr int kStageBytes = LBOX * (kXBytes + kABytes);
   static constexpr int kBarOff = kStages * kStageBytes;
   static constexpr int kNumBars = 2 * kStages + 4;   // full[S], empty[S], tfull[2], tempty[2]
-  static constexpr int kTmemCols = NC <= 32 ? 64 : (NC <= 64 ? 128 : 256);   // two accumulators, a power of two
+  static constexpr int kTmemCols = NC <= 32 ? 64 : (NC <= 64 ? 128 : 256);   // two accumulators, a power of two; per slice
   static constexpr int kMiscOff = kBarOff + kNumBars * 8;
   static constexpr int kDynamic = kMiscOff + 16 + 1024;
 };
@@ -54,7 +57,8 @@ template <typename T, int NC>
 __global__ void __launch_bounds__(kLowThreads, 1)
 pq_lowrank_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmX1,
                        const __grid_constant__ CUtensorMap tmA, T* __restrict__ t,
-                       int64_t ldt, int M, int K, int k0, int32_t* status) {
+                       int64_t ldt, int M, int K, int k0, int slice_kb, int slices, int32_t* status) {
+  // slices > 1 (NC == 32 only): slice i sums k-blocks [i slice_kb, (i + 1) slice_kb) in accumulator columns [32 i, +32)
   using L = LowSmem<NC>;
   constexpr int LSTAGES = L::kStages;
   extern __shared__ uint8_t smem_raw[];
@@ -70,7 +74,8 @@ pq_lowrank_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
   const int lane = threadIdx.x & 31;
   const int tiles = (M + LM - 1) / LM;
   const int num_kb = (K + LBOX * LKE - 1) / (LBOX * LKE);
-  constexpr uint32_t kTmemCols = L::kTmemCols;       // two accumulators of NC columns
+  uint32_t tmem_cols = L::kTmemCols;                 // two accumulators of NC columns per slice, a power of two
+  if (NC == 32) while (static_cast<int>(tmem_cols) < 2 * NC * slices) tmem_cols *= 2;
 
   if (threadIdx.x == 0) {
     tma_prefetch_desc(&tmX); tma_prefetch_desc(&tmX1); tma_prefetch_desc(&tmA);
@@ -80,7 +85,7 @@ pq_lowrank_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     fence_mbar_init();
     fence_proxy_async_smem();
   }
-  if (warp == 1) { tmem_alloc(tmem_holder, kTmemCols); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc(tmem_holder, tmem_cols); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -133,9 +138,13 @@ pq_lowrank_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
           report_timeout(status, 2, 2); *abort_flag = 1; ok = false; break;
         }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * NC);
+        uint32_t d_tmem = tmem_base + static_cast<uint32_t>(buf * NC * slices);
+        int left = slice_kb;                           // k-blocks left in this slice
 #pragma unroll 1
         for (int kb = 0; kb < num_kb; ++kb) {
+          if (left == 0) { d_tmem += NC; left = slice_kb; }
+          const bool fresh = left == slice_kb;
+          --left;
           if (!wait_or_abort(&full_bar[stage], phase, abort_flag)) {
             report_timeout(status, 2, 1); *abort_flag = 1; ok = false; break;
           }
@@ -148,7 +157,7 @@ pq_lowrank_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
 #pragma unroll
             for (int k = 0; k < LKE / 16; ++k)
               tc_mma_f16(d_tmem, a_desc + static_cast<uint64_t>(2 * k), b_desc + static_cast<uint64_t>(2 * k), idesc,
-                         (kb > 0 || b > 0 || k > 0) ? 1u : 0u);
+                         (!fresh || b > 0 || k > 0) ? 1u : 0u);
           }
           tc_commit(&empty_bar[stage]);
           if (++stage == LSTAGES) { stage = 0; phase ^= 1u; }
@@ -176,8 +185,22 @@ pq_lowrank_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
 #pragma unroll
       for (int cg = 0; cg < NC / 32; ++cg) {           // 32 columns at a time
         uint32_t v[32];
-        tmem_ld_32x32b_x32(tmem_base + static_cast<uint32_t>(buf * NC + cg * 32) + (static_cast<uint32_t>(quarter * 32) << 16), v);
+        const uint32_t t_addr = tmem_base + static_cast<uint32_t>(buf * NC * slices + cg * 32) + (static_cast<uint32_t>(quarter * 32) << 16);
+        tmem_ld_32x32b_x32(t_addr, v);
         tc_wait_ld();
+        if constexpr (NC == 32) {
+          // the slices in order, starting from zero, as the owner of a row adds them in quant_down.cu
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(0.0f + __uint_as_float(v[j]));
+#pragma unroll 1
+          for (int i = 1; i < slices; ++i) {
+            uint32_t u[32];
+            tmem_ld_32x32b_x32(t_addr + static_cast<uint32_t>(i * NC), u);
+            tc_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(u[j]));
+          }
+        }
         if (cg == NC / 32 - 1) {                       // the accumulator is in registers: the MMA thread may reuse it
           tc_fence_before();
           __syncwarp();
@@ -202,7 +225,7 @@ pq_lowrank_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
       for (int k = 0; k < 64; ++k) __nanosleep(1000);
     }
     tc_fence_after();
-    tmem_dealloc(tmem_base, kTmemCols);
+    tmem_dealloc(tmem_base, tmem_cols);
   }
 }
 
@@ -223,7 +246,7 @@ int make_map16(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int6
 
 template <typename T, int NC>
 int launch_low(const CUtensorMap& tmX, const CUtensorMap& tmX1, int k0, const CUtensorMap& tmA, void* t, int64_t ldt, int64_t M,
-               int64_t K, int32_t* status, cudaStream_t st) {
+               int64_t K, int slice_kb, int slices, int32_t* status, cudaStream_t st) {
   auto kern = pq_lowrank_down_kernel<T, NC>;
   using LS = LowSmem<NC>;
   static bool attr_set[64] = {false};
@@ -238,7 +261,7 @@ int launch_low(const CUtensorMap& tmX, const CUtensorMap& tmX1, int k0, const CU
   int64_t grid = sm_count();
   if (grid > tiles) grid = tiles;
   kern<<<static_cast<unsigned>(grid), kLowThreads, LS::kDynamic, st>>>(tmX, tmX1, tmA, static_cast<T*>(t), ldt,
-                                                                           static_cast<int>(M), static_cast<int>(K), k0, status);
+                                                                           static_cast<int>(M), static_cast<int>(K), k0, slice_kb, slices, status);
   PQ_CUDA_TRY(cudaGetLastError());
   return PQ_OK;
 }
@@ -246,11 +269,13 @@ int launch_low(const CUtensorMap& tmX, const CUtensorMap& tmX1, int k0, const CU
 template <typename T>
 int launch_low_cols(int R, const CUtensorMap& tmX, const CUtensorMap& tmX1, int k0, const CUtensorMap& tmA, void* t, int64_t ldt,
                     int64_t M, int64_t K, int32_t* status, cudaStream_t st) {
+  const int num_kb = static_cast<int>((K + LBOX * LKE - 1) / (LBOX * LKE));
+  const int slice_kb = R == 32 ? lowrank_slice_blocks(K) : num_kb, slices = (num_kb + slice_kb - 1) / slice_kb;
   switch (R) {
-    case 32: return launch_low<T, 32>(tmX, tmX1, k0, tmA, t, ldt, M, K, status, st);
-    case 64: return launch_low<T, 64>(tmX, tmX1, k0, tmA, t, ldt, M, K, status, st);
-    case 96: return launch_low<T, 96>(tmX, tmX1, k0, tmA, t, ldt, M, K, status, st);
-    case 128: return launch_low<T, 128>(tmX, tmX1, k0, tmA, t, ldt, M, K, status, st);
+    case 32: return launch_low<T, 32>(tmX, tmX1, k0, tmA, t, ldt, M, K, slice_kb, slices, status, st);
+    case 64: return launch_low<T, 64>(tmX, tmX1, k0, tmA, t, ldt, M, K, slice_kb, slices, status, st);
+    case 96: return launch_low<T, 96>(tmX, tmX1, k0, tmA, t, ldt, M, K, slice_kb, slices, status, st);
+    case 128: return launch_low<T, 128>(tmX, tmX1, k0, tmA, t, ldt, M, K, slice_kb, slices, status, st);
     default: return PQ_ERR_UNSUPPORTED;
   }
 }
@@ -277,8 +302,7 @@ int lowrank_down_impl(const void* x, int64_t K0, int64_t ldx, const void* x1, in
   if (K1 > 0 && (K1 % 8 != 0 || ldx1 % 8 != 0 || !aligned_to(x1, 16))) return PQ_ERR_ALIGN;
   if (K1 > 0 && K0 % LKE != 0) return PQ_ERR_UNSUPPORTED;       // the seam has to fall between two 64-element boxes
   if (workspace != nullptr && ws_bytes < PQ_GEMM_WORKSPACE_BYTES) return PQ_ERR_WORKSPACE;
-  // one factor and rows of a certain length: the cluster kernel, whose t the fused quantisation + down-projection repeats
-  if (lowrank_sliced(K, R))
+  if (lowrank_few_rows(M, K, R))
     return lowrank_down_sliced(x, K0, ldx, x1, K1, ldx1, dtype, a_t, lda, R, t, ldt, M, workspace, ws_bytes, stream);
   const bool bf16 = dtype == PQ_DTYPE_BF16;
   CUtensorMap tmX, tmX1, tmA;

@@ -492,6 +492,28 @@ int launch_qd_cl(int cl, const CUtensorMap& tmX, const CUtensorMap& tmX1, const 
 
 using namespace pq;
 
+namespace pq {
+namespace {
+// Cluster size, a function of K alone so that a row's t does not depend on how many rows it is computed with: slices of
+// at most twelve k-blocks (a 96 KB slice of A leaves the x ring six stages), sixteen with the largest cluster.  Slices of
+// six: 512 x 3072 9.0 instead of 12.4 us, but 4608 x 3072 17.9 instead of 14.8 us and 65536 x 6144 273 instead of 255 us.
+int cluster_size(int64_t K) {
+  const int64_t num_kb = (K + QKB - 1) / QKB;
+  int cl = 1;
+  while (cl < 8 && (num_kb + cl - 1) / cl > 12) cl *= 2;
+  return cl;
+}
+}  // namespace
+// k-blocks of 128 elements that are summed in one accumulator, here and in the streaming kernel of lowrank.cu (whose rows may
+// be longer than this kernel takes: those are one slice).
+int lowrank_slice_blocks(int64_t K) {
+  const int64_t num_kb = (K + QKB - 1) / QKB;
+  if (K > 8 * kSliceKbMax * QKB) return static_cast<int>(num_kb);
+  const int cl = cluster_size(K);
+  return static_cast<int>((num_kb + cl - 1) / cl);
+}
+}  // namespace pq
+
 namespace {
 // q == nullptr: t only
 int quant_down_impl(const void* x0, int64_t K0, int64_t ldx0, const void* x1, int64_t K1, int64_t ldx1, int dtype, int64_t M,
@@ -530,13 +552,8 @@ int quant_down_impl(const void* x0, int64_t K0, int64_t ldx0, const void* x1, in
   p.status = static_cast<int32_t*>(workspace);
   p.M = static_cast<int>(M); p.K = static_cast<int>(K);
   p.k0 = static_cast<int>(K1 > 0 ? K0 : K + QKB);               // one source: nothing comes from the second
-  const int num_kb = static_cast<int>((K + QKB - 1) / QKB);
-  // Cluster size, a function of K alone so that a row's t does not depend on how many rows it is computed with: slices of
-  // at most twelve k-blocks (a 96 KB slice of A leaves the x ring six stages), sixteen with the largest cluster.  Slices of
-  // six: 512 x 3072 9.0 instead of 12.4 us, but 4608 x 3072 17.9 instead of 14.8 us and 65536 x 6144 273 instead of 255 us.
-  int cl = 1;
-  while (cl < 8 && (num_kb + cl - 1) / cl > 12) cl *= 2;
-  p.kb_slice = (num_kb + cl - 1) / cl;
+  const int cl = cluster_size(K);
+  p.kb_slice = lowrank_slice_blocks(K);
   p.stages = 0;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (K1 > 0) {
@@ -549,10 +566,16 @@ int quant_down_impl(const void* x0, int64_t K0, int64_t ldx0, const void* x1, in
 }  // namespace
 
 namespace pq {
-// Where pq_lowrank_down takes this kernel: the row lengths for which quantisation and down-projection are one launch
-// (ops.QUANT_LOWRANK_K), so that t is the same bits whichever entry point computes it.  Against the streaming kernel of
-// lowrank.cu: 512 x 12288 23 -> 8.2 us, 4608 x 3072 9.8 -> 10.4 us, 66048 x 3072 68 -> 65 us, 66048 x 15360 306 -> 322 us.
+// Row lengths for which quantisation and down-projection are one launch (ops.QUANT_LOWRANK_K).
 bool lowrank_sliced(int64_t K, int R) { return R == QNC && K >= 512 && K <= 8 * kSliceKbMax * QKB; }
+// Where t alone is taken from this kernel: few and long rows, which leave most SMs without one of the streaming kernel's 64-row
+// tiles.  With enough tiles that kernel is ahead (six stages of x on every SM, no exchange).  Streaming / this one, us:
+// 512 x 3072 8.0 / 7.3, 2048 x 3072 8.8 / 8.6, 4608 x 3072 9.6 / 10.3, 2048 x 6144 13.8 / 9.9, 4608 x 6144 15.3 / 16.3,
+// 512 x 12288 22.9 / 8.6, 4608 x 12288 27.2 / 23.4, 8256 x 12288 36.3 / 37.3, 66048 x 15360 301 / 325; 512 x 1024 4.9 / 6.7.
+// The sums are the same bits either way.
+bool lowrank_few_rows(int64_t M, int64_t K, int R) {
+  return lowrank_sliced(K, R) && K >= 3072 && 2 * M <= K && M <= 32 * static_cast<int64_t>(sm_count());
+}
 int lowrank_down_sliced(const void* x0, int64_t K0, int64_t ldx0, const void* x1, int64_t K1, int64_t ldx1, int dtype,
                         const void* a_t, int64_t lda, int R, void* t, int64_t ldt, int64_t M, void* workspace, size_t ws_bytes,
                         void* stream) {

@@ -1292,6 +1292,32 @@ def test_quant_rows_lowrank(cuda_dev, M, K, K1, dtype):
         assert torch.equal(t[: M // 2], ops.quant_rows_lowrank(x0[: M // 2], a_t)[2])   # whatever the number of rows
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,K1", [(2500, 512, 0), (40, 1536, 0), (3001, 1544, 0), (40, 3072, 0), (1536, 3072, 0), (1537, 3072, 0),
+                                    (9700, 3072, 0), (130, 6152, 0), (4200, 6152, 0), (2200, 12288, 0), (9700, 15360, 0),
+                                    (4800, 16384, 0), (300, 16392, 0), (700, 3072, 6144), (5000, 1024, 520), (5000, 192, 72)])
+def test_lowrank_down_is_one_sum_in_every_kernel(cuda_dev, M, K, K1, dtype):
+    """t of a row is the same bits from the streaming kernel (many rows), from the cluster kernel (few long rows) and from the
+    one-launch quantisation + down-projection, whatever the number of rows, for one source and for two; a last column slice
+    that is short or missing, one to eight slices, rows beyond the one-launch form's length."""
+    g = torch.Generator(device="cuda").manual_seed(M + K + K1)
+    Kt = K + K1
+    x = torch.randn(M, Kt, generator=g, device=cuda_dev).to(dtype)
+    a_t = (torch.randn(32, Kt, generator=g, device=cuda_dev) * 0.05).to(dtype)
+    t = ops.lowrank_down(x, a_t)
+    if Kt <= 16384:
+        assert torch.equal(t, ops.quant_rows_lowrank(x, a_t)[2])
+    assert torch.equal(t[:33], ops.lowrank_down(x[:33], a_t)) and torch.equal(t[7:], ops.lowrank_down(x[7:], a_t))
+    if K1:
+        x0, x1 = x[:, :K].contiguous(), x[:, K:].contiguous()
+        assert torch.equal(t, ops.lowrank_down_cat(x0, x1, a_t)) and torch.equal(t, ops.quant_rows_lowrank(x0, a_t, x1)[2])
+        assert torch.equal(t[:33], ops.lowrank_down_cat(x0[:33], x1[:33], a_t))
+    ref, mag = x.double() @ a_t.double().t(), x.double().abs() @ a_t.double().abs().t()
+    ulp = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert bool(((t.double() - ref).abs() <= ulp * ref.abs() * 1.01 + 1e-6 * mag).all())
+    ops.check_device_status(cuda_dev)
+
+
 # ------------------------------------------------------------------------------------------------ whole forward in one call
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("M,K,N,lowrank", [(1, 64, 8, False), (154, 640, 1280, False), (77, 1808, 2376, False),
