@@ -356,9 +356,9 @@ class Int8Linear(nn.Module):
         return t if t is not None else getattr(self, name)
 
     def _lean_forward(self, x2: torch.Tensor):
-        """Eager fast path for the common case (aligned rows, no branch or a rank-32 one whose down-projection shares the
-        quantisation's launch): one C-ABI call with the per-layer constants in a descriptor, skipping the generic wrappers'
-        checks.  Returns None when the input does not qualify."""
+        """Eager fast path for the common case (aligned rows, no branch or a rank-32 one): one C-ABI call with the per-layer
+        constants in a descriptor, skipping the generic wrappers' checks; for rows whose down-projection does not share the
+        quantisation's launch the three calls are made from here.  Returns None when the input does not qualify."""
         M, K = x2.shape
         dt = x2.dtype
         w = self._operand("weight_int8")
@@ -367,18 +367,19 @@ class Int8Linear(nn.Module):
             return None
         lr_a, bias = self._operand("lr_A"), self._operand("bias")
         rank = 0
+        low = None
+        one_launch = True
         if lr_a is not None:
-            if not self._fusable_lowrank(x2) or not ops.quant_lowrank_ok(x2):
+            if not self._fusable_lowrank(x2):
                 return None
             rank = 32
-            lr_b, lbt, at = self.lr_B, self._lr_Bt(), self._lr_At()
+            one_launch = ops.quant_lowrank_ok(x2)              # else: rows too short or too long for the shared launch
+            lr_b, lbt, at = self.lr_B, self._lr_Bt(), self._lr_At() if one_launch else None
             # the library sees bare pointers: factors that do not fit the layer must not get there
-            assert at.shape == (32, K) and at.device == x2.device, (tuple(at.shape), at.device)
+            assert at is None or (at.shape == (32, K) and at.device == x2.device), (tuple(at.shape), at.device)
             if lr_b.stride(1) != 1:
                 return None
-            low = (lr_b.data_ptr(), lbt.data_ptr(), at.data_ptr())
-        else:
-            low = None
+            low = (lr_b.data_ptr(), lbt.data_ptr(), at.data_ptr() if one_launch else None)
         # every buffer whose address is cached takes part in the key: .to(dtype) / .half() / load_state_dict(assign=True)
         # replace the float buffers while the int8 weight stays where it is
         sc = self._operand("w_scale")
@@ -401,13 +402,27 @@ class Int8Linear(nn.Module):
             # the library, the descriptor and its address, and what the addresses in it belong to
             c = (key, ops._LIB().pq_int8_linear, d, ctypes.addressof(d), N, K, ws)
             self.__dict__["_lean_cache"] = c
-        _key, call, _d, d_ptr, N, K_w, _ws = c
+        _key, call, d, d_ptr, N, K_w, ws = c
         assert K == K_w, (K, K_w)
+        ldx = x2.stride(0) if M > 1 else K
+        if not one_launch:
+            t = self._down(x2)
+            q, sx, out = x2.new_empty((M, K), dtype=torch.int8), x2.new_empty((M,), dtype=torch.float32), x2.new_empty((M, N))
+            lib, code, stream = ops._LIB(), d.dtype, ops._stream(x2)
+            with ops._on_device(x2):
+                rc = lib.pq_quant_rows(x2.data_ptr(), code, M, K, ldx, q.data_ptr(), sx.data_ptr(), stream)
+                if rc == 0:
+                    rc = lib.pq_int8_gemm(q.data_ptr(), K, sx.data_ptr(), d.w, d.ldw, d.s_col, d.bias, t.data_ptr(), t.stride(0),
+                                          d.lb, d.ldb, d.lb_t, rank, code, out.data_ptr(), code, N, M, N, K, d.workspace,
+                                          d.ws_bytes, None, stream)
+            if rc:
+                ops._lib.check(rc, f"Int8Linear(M={M}, N={N}, K={K})")
+            return out
         nbytes = ops.linear_scratch_bytes(M, K, rank)
         scratch = x2.new_empty((nbytes,), dtype=torch.uint8)
         out = x2.new_empty((M, N))
         with ops._on_device(x2):
-            rc = call(d_ptr, x2.data_ptr(), x2.stride(0) if M > 1 else K, M, scratch.data_ptr(), nbytes, out.data_ptr(), N,
+            rc = call(d_ptr, x2.data_ptr(), ldx, M, scratch.data_ptr(), nbytes, out.data_ptr(), N,
                       ops._stream(x2))
         if rc:
             ops._lib.check(rc, f"Int8Linear(M={M}, N={N}, K={K})")

@@ -1354,6 +1354,23 @@ def test_linear_in_one_call(cuda_dev, M, K, N, lowrank, dtype):
                                                            bare.lr_B, dtype))
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K", [(1, 32), (70, 256), (70, 480), (70, 512), (70, 16384), (70, 16416)])
+def test_linear_fast_path_at_every_row_length(cuda_dev, M, K, dtype):
+    """A rank-32 layer takes the fast path whether or not its down-projection shares the quantisation's launch (rows of 512 to
+    16384 features), bit-equal to the separate operators, also on a row-strided input."""
+    g = torch.Generator().manual_seed(M + K)
+    N = 264
+    m = _toy_layer(cuda_dev, g, K, N, lowrank=True, dtype=dtype)
+    wide = rand_act(M, K + 24, dtype, M + 11).to(cuda_dev)
+    for x in (wide[:, :K].contiguous(), wide[:, :K]):
+        y = m(x)
+        assert "_lean_cache" in m.__dict__
+        xq, sx = int8_exec.quant_rows(x)
+        assert torch.equal(y, int8_exec.int8_gemm_lr(xq, sx, m.weight_int8, m.w_scale, m.bias, m._down(x), m.lr_B, dtype))
+    ops.check_device_status(cuda_dev)
+
+
 class _Doubled(nn.Module):
     def forward(self, t):
         return t * 2
