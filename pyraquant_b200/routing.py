@@ -142,9 +142,10 @@ class RoutePlan:
         return int(self.row_idx.shape[0])
 
     def untouched(self) -> np.ndarray:
-        """int32: the canvas tokens without a contributor, ascending."""
+        """int32: the canvas tokens without a contributor, ascending.  Entries of ``tokens`` outside the canvas, which the
+        kernels skip, name no token."""
         mask = np.ones(int(self.token_hw[0]) * int(self.token_hw[1]), dtype=bool)
-        mask[self.tokens] = False
+        mask[self.tokens[(self.tokens >= 0) & (self.tokens < mask.size)]] = False
         return np.flatnonzero(mask).astype(np.int32)
 
     def to(self, device) -> Dict[str, torch.Tensor]:
@@ -306,7 +307,8 @@ def fuse_rows(background: torch.Tensor, y: torch.Tensor, plan: RoutePlan) -> tor
             and bg.stride(1) == 1 and bg.stride(0) % 8 == 0 and bg.data_ptr() % 16 == 0 and y.dim() == 2 and y.stride(1) == 1
             and y.stride(0) % 8 == 0 and y.data_ptr() % 16 == 0 and (H, W) == tuple(plan.token_hw)):
         d = plan.to(bg.device)
-        if d["tokens"].numel() + d["rest"].numel() == H * W:          # a hand-made plan may list a token twice
+        # a hand-made plan may list a token twice, or one outside the canvas: every row is then not listed exactly once
+        if d["tokens"].numel() + d["rest"].numel() == H * W:
             return ops.fuse_rows(bg, y, d["tokens"], d["ptr"], d["src"], d["beta"], d["rest"]).reshape(1, H, W, C)
     out = bg.clone()
     scatter_rows_(y, plan, out)

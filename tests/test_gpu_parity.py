@@ -1464,3 +1464,29 @@ def test_fuse_rows_out_of_place(cuda_dev, dtype, hw, C, halo, boxes):
         assert got.shape == (1, H, W, C)
         assert torch.equal(got.reshape(H * W, C).view(torch.int16), want.view(torch.int16))
         assert torch.equal(bg, before)
+
+
+@pytest.mark.parametrize("extra", [[-1], [64, 2 ** 30], [5], [-3, 5, 64]])
+def test_fuse_rows_with_a_hand_made_token_list(cuda_dev, extra):
+    """Tokens outside the canvas are skipped and a token listed twice is blended as the in-place scatter blends it; every other
+    row is the background's."""
+    tokens = np.array([3, 5, 40] + extra, np.int32)
+    n = tokens.size
+    beta = np.full(n, 0.5, np.float32)
+    plan = routing.RoutePlan(token_hw=(8, 8), patches=[], bucket_shapes=[], row_idx=np.arange(n, dtype=np.int32), m_hi=n,
+                             tokens=tokens, ptr=np.arange(n + 1, dtype=np.int32), src=np.arange(n, dtype=np.int32), beta=beta)
+    if extra.count(5):                                    # twice in one launch: the order is open, so both do the same
+        plan.beta[:] = 1.0
+        plan.src[:] = 0
+    g = torch.Generator().manual_seed(n)
+    bg = torch.randn(1, 8, 8, 64, generator=g).to(torch.bfloat16).to(cuda_dev)
+    y = torch.randn(n, 64, generator=g).to(torch.bfloat16).to(cuda_dev)
+    want = bg.reshape(64, 64).clone()
+    inside = [i for i, t in enumerate(tokens) if 0 <= t < 64]
+    routing.scatter_rows_(y, routing.RoutePlan(
+        token_hw=(8, 8), patches=[], bucket_shapes=[], row_idx=plan.row_idx, m_hi=n, tokens=tokens[inside],
+        ptr=np.arange(len(inside) + 1, dtype=np.int32), src=plan.src[inside], beta=plan.beta[inside]), want)
+    torch.empty(64, 64, dtype=torch.bfloat16, device=cuda_dev).fill_(float("nan"))     # what a row left unwritten would hold
+    assert torch.equal(routing.fuse_rows(bg, y, plan).reshape(64, 64), want)
+    canvas = bg.reshape(64, 64).clone()
+    assert torch.equal(routing.scatter_rows_(y, plan, canvas), want)

@@ -288,3 +288,17 @@ def test_pack_int4_layout():
     assert p.tolist() == [[0x78, 0xF0, 0xC3, 0x21]]
     with pytest.raises(AssertionError):
         ops.pack_int4(torch.tensor([[8, 0]], dtype=torch.int8))
+
+
+@pytest.mark.parametrize("extra", [[], [-1], [-7, 3], [64], [10 ** 6], [5, 5]])
+def test_untouched_tokens_of_a_hand_made_plan(extra):
+    """Entries outside the canvas name no token (the kernels skip them), and touched and untouched tokens together count the
+    canvas only where every row is listed exactly once: the out-of-place fusion relies on that."""
+    tokens = np.array([3, 5, 40] + extra, np.int32)
+    n = tokens.size
+    plan = routing.RoutePlan(token_hw=(8, 8), patches=[], bucket_shapes=[], row_idx=np.arange(n, dtype=np.int32), m_hi=n,
+                             tokens=tokens, ptr=np.arange(n + 1, dtype=np.int32), src=np.arange(n, dtype=np.int32),
+                             beta=np.ones(n, np.float32))
+    assert plan.untouched().tolist() == [t for t in range(64) if t not in (3, 5, 40)]
+    d = plan.to("cpu")
+    assert (d["tokens"].numel() + d["rest"].numel() == 64) == (not extra)
