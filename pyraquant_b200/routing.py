@@ -297,6 +297,11 @@ def scatter_rows_(y: torch.Tensor, plan: RoutePlan, canvas: torch.Tensor) -> tor
     return canvas
 
 
+def _tracked(t: torch.Tensor) -> bool:
+    """Whether autograd follows `t` (backward graph or forward-mode tangent), so that a copy of it is torch's to make."""
+    return (t.requires_grad and torch.is_grad_enabled()) or torch.autograd.forward_ad.unpack_dual(t).tangent is not None
+
+
 def fuse_rows(background: torch.Tensor, y: torch.Tensor, plan: RoutePlan) -> torch.Tensor:
     """Out-of-place form with the reference's calling shape: background [1,H,W,C] -> fused [1,H,W,C]."""
     b, H, W, C = background.shape
@@ -305,7 +310,7 @@ def fuse_rows(background: torch.Tensor, y: torch.Tensor, plan: RoutePlan) -> tor
     bg = background.reshape(H * W, C)
     if (_eager() and bg.is_cuda and y.device == bg.device and y.dtype == bg.dtype and y.dtype in ops._DT and C % 8 == 0
             and bg.stride(1) == 1 and bg.stride(0) % 8 == 0 and bg.data_ptr() % 16 == 0 and y.dim() == 2 and y.stride(1) == 1
-            and y.stride(0) % 8 == 0 and y.data_ptr() % 16 == 0 and (H, W) == tuple(plan.token_hw)):
+            and y.stride(0) % 8 == 0 and y.data_ptr() % 16 == 0 and (H, W) == tuple(plan.token_hw) and not _tracked(bg)):
         d = plan.to(bg.device)
         # a hand-made plan may list a token twice, or one outside the canvas: every row is then not listed exactly once
         if d["tokens"].numel() + d["rest"].numel() == H * W:

@@ -1490,3 +1490,25 @@ def test_fuse_rows_with_a_hand_made_token_list(cuda_dev, extra):
     assert torch.equal(routing.fuse_rows(bg, y, plan).reshape(64, 64), want)
     canvas = bg.reshape(64, 64).clone()
     assert torch.equal(routing.scatter_rows_(y, plan, canvas), want)
+
+
+def test_fuse_rows_keeps_the_background_in_the_graph(cuda_dev):
+    """The result carries the background's gradient and its forward-mode tangent, as a clone of it does; the values are those of
+    an untracked background."""
+    import torch.autograd.forward_ad as fwad
+    plan = routing.build_route_plan((8, 8), [(0, 4, 0, 4)], 1)
+    g = torch.Generator().manual_seed(5)
+    bg = torch.randn(1, 8, 8, 64, generator=g).to(torch.bfloat16).to(cuda_dev)
+    y = torch.randn(plan.n_rows, 64, generator=g).to(torch.bfloat16).to(cuda_dev)
+    want = routing.fuse_rows(bg, y, plan)
+    tracked = bg.clone().requires_grad_()
+    got = routing.fuse_rows(tracked, y, plan)
+    assert got.requires_grad and torch.equal(got.detach(), want)
+    got.sum().backward()
+    assert torch.equal(tracked.grad, torch.ones_like(bg))
+    with torch.no_grad():
+        assert torch.equal(routing.fuse_rows(tracked, y, plan), want)
+    with fwad.dual_level():
+        dual = fwad.make_dual(bg, torch.ones_like(bg))
+        out = fwad.unpack_dual(routing.fuse_rows(dual, y, plan))
+        assert torch.equal(out.primal, want) and out.tangent is not None
