@@ -23,7 +23,8 @@ extern "C" int pq_int8_linear(const pq_linear_desc* d, const void* x, int64_t ld
                               int64_t scratch_bytes, void* out, int64_t ldo, void* stream) {
   if (d == nullptr) return PQ_ERR_NULL;
   if (M < 0 || d->N <= 0 || d->K <= 0) return PQ_ERR_SHAPE;
-  if (d->rank != 0 && !lowrank_sliced(d->K, d->rank)) return PQ_ERR_UNSUPPORTED;
+  if (d->rank != 0 && (!lowrank_sliced(d->K, d->rank) || d->lb == nullptr || d->lb_t == nullptr || d->a_t == nullptr))
+    return PQ_ERR_UNSUPPORTED;
   if (M == 0) return PQ_OK;
   if (scratch == nullptr) return PQ_ERR_NULL;
   if (!aligned_to(scratch, 256)) return PQ_ERR_ALIGN;

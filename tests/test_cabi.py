@@ -178,6 +178,64 @@ def test_scatter_and_gather_argument_checks():
     assert lib.pq_int8_gemm_g32(p16, 128, None, p16, 128, p16, None, p16, 0, 64, 8, 64, 128, None, 0, None) == 1
 
 
+def test_one_launch_and_one_call_argument_checks():
+    """The fused entry points refuse bad calls before anything is launched: absent operands, seams and row lengths the kernels
+    do not take, misaligned or too little scratch."""
+    lib = _lib.load()
+    buf = ctypes.create_string_buffer(8192)
+    p16 = (ctypes.addressof(buf) + 255) & ~255
+
+    def ql(x0=p16, K0=512, ldx0=512, x1=None, K1=0, ldx1=0, dtype=0, M=4, a=p16, lda=512, R=32, q=p16, s=p16, t=p16, ldt=32, ws=None,
+           ws_bytes=0):
+        return lib.pq_quant_rows_lowrank(x0, K0, ldx0, x1, K1, ldx1, dtype, M, a, lda, R, q, s, t, ldt, ws, ws_bytes, None)
+
+    assert ql(M=0) == 0
+    assert ql(x0=None) == ql(a=None) == ql(q=None) == ql(s=None) == ql(t=None) == 1
+    assert ql(K1=64, ldx1=64, lda=576) == 1           # second source announced but absent
+    assert ql(K0=0) == ql(ldx0=504) == ql(lda=504) == ql(ldt=16) == ql(M=-1) == ql(x1=p16, K1=64, ldx1=8, lda=576) == 2
+    assert ql(K0=508, ldx0=512) == ql(ldx0=516) == ql(x0=p16 + 2) == ql(t=p16 + 8) == ql(q=p16 + 4) == ql(s=p16 + 2) == 3
+    assert ql(dtype=5) == 4
+    assert ql(R=64, lda=512, ldt=64) == ql(K0=16392, ldx0=16392, lda=16392) == 7
+    assert ql(x1=p16, K0=480, K1=64, ldx1=64, lda=544) == 7          # seam off the 64-element grid
+    assert ql(ws=p16, ws_bytes=8) == 8
+
+    def linear(x=p16, ldx=512, M=4, scratch=p16, nbytes=8192, out=p16, ldo=64, d="default", **kw):
+        f = dict(w=p16, s_col=p16, bias=None, lb=p16, lb_t=p16, a_t=p16, ldw=512, ldb=64, N=64, K=512, workspace=None, ws_bytes=0,
+                 rank=32, dtype=0)
+        f.update(kw)
+        desc = _lib.LinearDesc(**f)
+        return lib.pq_int8_linear(ctypes.addressof(desc) if d is not None else None, x, ldx, M, scratch, nbytes, out, ldo, None)
+
+    need = lib.pq_int8_linear_scratch_bytes(4, 512, 32)
+    assert need == 4 * 512 + 256 + 256
+    assert linear(M=0) == 0
+    assert linear(d=None) == linear(scratch=None) == 1
+    assert linear(M=-1) == linear(N=0) == linear(K=0) == 2
+    assert linear(scratch=p16 + 16) == 3
+    assert linear(rank=16) == linear(K=256, ldx=256) == linear(K=16416, ldx=16416) == 7
+    assert linear(lb=None) == linear(lb_t=None) == linear(a_t=None) == 7
+    assert linear(nbytes=need - 1) == 8
+    assert linear(x=None) == 1 and linear(x=None, rank=0) == 1
+    assert lib.pq_int8_linear_scratch_bytes(-1, 512, 32) == 0
+
+    def g32(x=p16, M=4, N=64, K=128, scratch=p16, nbytes=8192):
+        return lib.pq_int8_linear_g32(x, 0, K, p16, K, p16, None, scratch, nbytes, p16, N, M, N, K, None, 0, None)
+
+    assert g32(M=0) == 0
+    assert g32(scratch=None) == g32(x=None) == 1
+    assert g32(N=0) == 2 and g32(scratch=p16 + 16) == 3 and g32(K=96) == 7
+    assert g32(nbytes=lib.pq_int8_linear_g32_scratch_bytes(4, 128) - 1) == 8
+
+    def fuse(y=p16, ldy=64, tokens=p16, rest=p16, n_tokens=2, n_rest=2, bg=p16, out=p16, ldo=64, C=64, dtype=0):
+        return lib.pq_fuse_rows(y, ldy, 4, tokens, p16, p16, p16, n_tokens, rest, n_rest, bg, 64, out, ldo, 4, C, dtype, None)
+
+    assert fuse(n_tokens=0, n_rest=0) == 0
+    assert fuse(y=None) == fuse(tokens=None) == fuse(rest=None) == fuse(bg=None) == fuse(out=None) == 1
+    assert fuse(ldo=32) == fuse(n_rest=-1) == 2
+    assert fuse(C=60) == fuse(out=p16 + 8) == fuse(ldy=68) == 3
+    assert fuse(dtype=9) == 4
+
+
 def test_operand_extent_checks_run_on_the_host():
     """The C ABI sees bare pointers; the Python operators check every operand's extent before a launch, so a short
     scale, bias or low-rank tensor is an AssertionError instead of an out-of-bounds device read."""
