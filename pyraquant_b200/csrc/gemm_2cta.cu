@@ -10,8 +10,8 @@
 // Synchronisation.  "full" barriers live in CTA 0 and count the bytes of both CTAs' copies (CTA 1's TMA instructions
 // name CTA 0's barrier).  Everything the MMA thread publishes ("stage free", "accumulator complete", "low-rank MMAs
 // done") is committed twice, once to each CTA's copy of the barrier.  What the MMA thread waits for from the
-// epilogues ("accumulator drained", "scaled accumulator written back") is one barrier in CTA 0 with 16 arrivals, the
-// eight epilogue warps of CTA 1 arriving remotely.  Every wait is bounded; a wait that gives up records a code in the
+// epilogues ("accumulator drained", "scaled accumulator written back") is one barrier in CTA 0 with an arrival per
+// epilogue warp of the pair, those of CTA 1 arriving remotely.  Every wait is bounded; a wait that gives up records a code in the
 // status word, raises its CTA's abort flag and lets the CTA drain; the peer then runs into its own limits.  Both
 // CTAs meet at a cluster barrier before they exit so that neither leaves while its peer may still signal it.
 #include <type_traits>
@@ -62,21 +62,6 @@ struct PairSmem {
 // ---------------------------------------------------------------------------------------------
 // cluster / pair primitives
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_cta_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// shared::cluster address of `smem_addr` (an address of the executing CTA) in CTA `rank` of the cluster
-__device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
-  return r;
-}
 // Arrival on a barrier of either CTA of the pair.  What the arrival publishes lives in tensor memory or registers and
 // is ordered by tcgen05.wait / tcgen05.fence, so the default (CTA-scope release) form is used: a cluster-scope
 // release would make the warp wait for its outstanding global stores to be acknowledged first.
@@ -144,10 +129,6 @@ __device__ __forceinline__ uint64_t kmajor_sw64_desc(uint32_t smem_addr) {
   d |= static_cast<uint64_t>(1) << 46;
   d |= static_cast<uint64_t>(4) << 61;
   return d;
-}
-__host__ __device__ constexpr uint32_t idesc_f16(int M, int N, bool bf16) {
-  return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | (static_cast<uint32_t>(N >> 3) << 17) |
-         (static_cast<uint32_t>(M >> 4) << 24);
 }
 __device__ __forceinline__ void tmem_st_x8(uint32_t taddr, const uint32_t (&v)[32]) {
   asm volatile(
@@ -437,7 +418,7 @@ pq_int8_gemm_fused_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __
     // Per tile and column chunk: wait until all sixteen epilogue warps of the pair have written the scaled chunk back
     // to tensor memory, add t @ lbT on top with two kind::f16 MMAs (K = 16 each), publish "chunk complete" to both CTAs.
     if (elect_one()) {
-      constexpr uint32_t idesc_lr = idesc_f16(2 * BM, kLrChunkN, std::is_same<OutT, __nv_bfloat16>::value);
+      constexpr uint32_t idesc_lr = make_idesc_f16(2 * BM, kLrChunkN, std::is_same<OutT, __nv_bfloat16>::value);
       int it = 0, lb_col = -1; uint32_t lb_count = 0; bool ok = true;
       long long tm_det[2] = {0, 0};
       auto commit_both = [&](uint64_t* bar) { tc_commit_pair(smem_u32(bar)); tc_commit_pair(peer_addr(bar)); };

@@ -41,18 +41,6 @@ struct LowSmem {
   static constexpr int kDynamic = kMiscOff + 16 + 1024;
 };
 
-__device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-      : "memory");
-}
-__host__ __device__ constexpr uint32_t idesc_f16_f32acc(int M, int N, bool bf16) {
-  return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | (static_cast<uint32_t>(N >> 3) << 17) |
-         (static_cast<uint32_t>(M >> 4) << 24);
-}
-
 template <typename T, int NC>
 __global__ void __launch_bounds__(kLowThreads, 1)
 pq_lowrank_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmX1,
@@ -129,7 +117,7 @@ pq_lowrank_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (elect_one()) {
-      constexpr uint32_t idesc = idesc_f16_f32acc(LM, NC, std::is_same<T, __nv_bfloat16>::value);
+      constexpr uint32_t idesc = make_idesc_f16(LM, NC, std::is_same<T, __nv_bfloat16>::value);
       int stage = 0; uint32_t phase = 0; int it = 0; bool ok = true;
 #pragma unroll 1
       for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++it) {
@@ -227,21 +215,6 @@ pq_lowrank_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_con
     tc_fence_after();
     tmem_dealloc(tmem_base, tmem_cols);
   }
-}
-
-// 16-bit matrix [rows, K] with row stride ld elements; box = 64 elements (128 bytes) x box_rows, 128-byte swizzle.
-int make_map16(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_t ld, int box_rows, bool bf16) {
-  EncodeTiledFn fn = encode_fn();
-  if (fn == nullptr) return PQ_ERR_CUDA;
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(LKE), static_cast<cuuint32_t>(box_rows)};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
-                  const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) { g_last_cuda_error = static_cast<int>(r); return PQ_ERR_CUDA; }
-  return PQ_OK;
 }
 
 template <typename T, int NC>

@@ -66,28 +66,14 @@ struct QuantDownParams {
   int stages;
 };
 
-__device__ __forceinline__ uint32_t qd_cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t qd_cluster_id() {
+__device__ __forceinline__ uint32_t cluster_id() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%clusterid.x;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ uint32_t qd_num_clusters() {
+__device__ __forceinline__ uint32_t num_clusters() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%nclusterid.x;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void qd_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t qd_map(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
 __device__ __forceinline__ void st_async_b32(uint32_t addr, uint32_t v, uint32_t bar) {
@@ -97,18 +83,6 @@ __device__ __forceinline__ void st_async_v4(uint32_t addr, uint32_t a, uint32_t 
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1,%2,%3,%4}, [%5];"
                ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d), "r"(bar) : "memory");
 }
-__device__ __forceinline__ void qd_mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-      : "memory");
-}
-__host__ __device__ constexpr uint32_t qd_idesc(bool bf16) {      // fp32 accumulator, M = 64, N = 32, both K-major
-  return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | (static_cast<uint32_t>(QNC >> 3) << 17) |
-         (static_cast<uint32_t>(QM >> 4) << 24);
-}
-
 // Shared memory: [A slice | x ring | t_in[2][CL][64 / CL][32] | amax_in[2][CL][64] | barriers]
 template <int CL>
 struct QDSmem {
@@ -149,7 +123,7 @@ pq_quant_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = qd_cluster_rank();
+  const uint32_t rank = cluster_cta_rank();
   const int blocks = (p.M + QM - 1) / QM;
   const int num_kb = (p.K + QKB - 1) / QKB;
   const int kb0 = static_cast<int>(rank) * p.kb_slice;
@@ -176,10 +150,10 @@ pq_quant_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   if (warp == 1) { tmem_alloc(tmem_holder, 64); tmem_relinquish(); }
   tc_fence_before();
   __syncthreads();
-  qd_cluster_sync();                                 // every CTA's barriers exist before anyone sends to them
+  cluster_sync_all();                                 // every CTA's barriers exist before anyone sends to them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
-  const int first = static_cast<int>(qd_cluster_id()), step = static_cast<int>(qd_num_clusters());
+  const int first = static_cast<int>(cluster_id()), step = static_cast<int>(num_clusters());
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -224,7 +198,7 @@ pq_quant_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
     if (my_kb > 0 && elect_one()) {
-      constexpr uint32_t idesc = qd_idesc(std::is_same<T, __nv_bfloat16>::value);
+      constexpr uint32_t idesc = make_idesc_f16(QM, QNC, std::is_same<T, __nv_bfloat16>::value);
       int stage = 0; uint32_t phase = 0; int it = 0; bool ok = true;
       if (!wait_or_abort(a_full, 0u, abort_flag)) { report_timeout(p.status, 2, 3); *abort_flag = 1; ok = false; }
 #pragma unroll 1
@@ -247,7 +221,7 @@ pq_quant_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             const uint64_t b_desc = make_kmajor_sw128_desc(smem_u32(smem + (2 * kb + b) * kQABoxBytes));
 #pragma unroll
             for (int k = 0; k < QKE / 16; ++k)
-              qd_mma_f16(d_tmem, a_desc + static_cast<uint64_t>(2 * k), b_desc + static_cast<uint64_t>(2 * k), idesc,
+              tc_mma_f16(d_tmem, a_desc + static_cast<uint64_t>(2 * k), b_desc + static_cast<uint64_t>(2 * k), idesc,
                          (kb > 0 || b > 0 || k > 0) ? 1u : 0u);
           }
           tc_commit(&empty_bar[stage]);
@@ -318,7 +292,7 @@ pq_quant_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       if (quant) {
         const uint32_t dst = smem_u32(max_in + (buf * CL + static_cast<int>(rank)) * QM + row), bar = smem_u32(&max_full[buf]);
 #pragma unroll
-        for (int k = tid & 1; k < CL; k += 2) st_async_b32(qd_map(dst, k), __float_as_uint(amax), qd_map(bar, k));
+        for (int k = tid & 1; k < CL; k += 2) st_async_b32(map_to_cta(dst, k), __float_as_uint(amax), map_to_cta(bar, k));
       }
       if (it > 0) {
         if (!finish_t(blk - step, it - 1)) { ok = false; break; }
@@ -348,8 +322,8 @@ pq_quant_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
       if (lane < 16) {
         const int r = quarter * 16 + lane;
         const uint32_t owner = static_cast<uint32_t>(r / kOwnRows);
-        const uint32_t dst = qd_map(smem_u32(t_in + ((buf * CL + static_cast<int>(rank)) * kOwnRows + r % kOwnRows) * QNC), owner);
-        const uint32_t bar = qd_map(smem_u32(&t_full[buf]), owner);
+        const uint32_t dst = map_to_cta(smem_u32(t_in + ((buf * CL + static_cast<int>(rank)) * kOwnRows + r % kOwnRows) * QNC), owner);
+        const uint32_t bar = map_to_cta(smem_u32(&t_full[buf]), owner);
 #pragma unroll
         for (int j = 0; j < 8; ++j) st_async_v4(dst + 16 * j, v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3], bar);
       }
@@ -416,26 +390,11 @@ pq_quant_down_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
   if (*abort_flag != 0) {
     for (int k = 0; k < 64; ++k) __nanosleep(1000);
   }
-  qd_cluster_sync();                                 // nobody leaves while its peers may still send to it
+  cluster_sync_all();                                 // nobody leaves while its peers may still send to it
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 64);
   }
-}
-
-// 16-bit matrix [rows, K], row stride ld elements; box = 64 elements x box_rows, 128-byte swizzle, zero fill.
-int qd_map16(CUtensorMap* map, const void* base, int64_t rows, int64_t K, int64_t ld, int box_rows, bool bf16) {
-  EncodeTiledFn fn = encode_fn();
-  if (fn == nullptr) return PQ_ERR_CUDA;
-  cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
-  cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * 2};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(QKE), static_cast<cuuint32_t>(box_rows)};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
-                  const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) { g_last_cuda_error = static_cast<int>(r); return PQ_ERR_CUDA; }
-  return PQ_OK;
 }
 
 constexpr int kQDMaxSmem = 232448;
@@ -534,15 +493,15 @@ int quant_down_impl(const void* x0, int64_t K0, int64_t ldx0, const void* x1, in
   if (workspace != nullptr && ws_bytes < PQ_GEMM_WORKSPACE_BYTES) return PQ_ERR_WORKSPACE;
   const bool bf16 = dtype == PQ_DTYPE_BF16;
   CUtensorMap tmX, tmX1, tmA;
-  int rc = qd_map16(&tmX, x0, M, K0, ldx0, QM, bf16);
+  int rc = make_map16(&tmX, x0, M, K0, ldx0, QM, bf16);
   if (rc != PQ_OK) return rc;
   if (K1 > 0) {
-    rc = qd_map16(&tmX1, x1, M, K1, ldx1, QM, bf16);
+    rc = make_map16(&tmX1, x1, M, K1, ldx1, QM, bf16);
     if (rc != PQ_OK) return rc;
   } else {
     tmX1 = tmX;
   }
-  rc = qd_map16(&tmA, a_t, R, K, lda, QNC, bf16);
+  rc = make_map16(&tmA, a_t, R, K, lda, QNC, bf16);
   if (rc != PQ_OK) return rc;
 
   QuantDownParams p;
