@@ -302,3 +302,56 @@ def test_untouched_tokens_of_a_hand_made_plan(extra):
     assert plan.untouched().tolist() == [t for t in range(64) if t not in (3, 5, 40)]
     d = plan.to("cpu")
     assert (d["tokens"].numel() + d["rest"].numel() == 64) == (not extra)
+
+
+def _rn32(hi, lo):
+    """The float32 nearest to hi + lo (a float64 sum and its exact error): rounded to odd first, so that the second rounding is
+    the only one that counts."""
+    even = (hi.view(np.int64) & 1) == 0
+    return np.where((lo != 0) & even, np.nextafter(hi, np.copysign(np.inf, lo)), hi).astype(np.float32)
+
+
+def _fma32(a, b, c):
+    """Correctly rounded float32 a * b + c (the float64 product of two float32 is exact)."""
+    p, c = a.astype(np.float64) * b.astype(np.float64), c.astype(np.float64)
+    s = p + c
+    t = s - p
+    return _rn32(s, (p - (s - t)) + (c - t))
+
+
+def _corrected_codes(x, amax):
+    """Codes of the kernels' quotient: product with the rounded reciprocal, exact residual, one correction, magic-number rounding."""
+    scale = np.maximum(amax, np.float32(1e-8)) / np.float32(127)
+    inv = np.float32(1) / scale
+    q0 = x * inv
+    q = _fma32(_fma32(-q0, np.broadcast_to(scale, x.shape), x), np.broadcast_to(inv, x.shape), q0)
+    m = q + np.float32(12582912.0)
+    want = np.clip(np.rint(x / scale), -127, 127).astype(np.int32)
+    return (m.view(np.int32) & 0xFF).astype(np.uint8).view(np.int8).astype(np.int32), want
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+def test_corrected_quotient_gives_the_codes_of_the_division(dtype):
+    """Every significand of the absmax with every value of the ten binades up to it, which covers all finite pairs: quotient and
+    correction scale exactly with a power of two (no operand underflows above the 1e-8 floor of the scale), and below
+    absmax / 1024 every code is 0.  Below the floor, every value of the type at the floor's scale."""
+    if dtype == "bf16":
+        val = lambda bits: (bits.astype(np.uint32) << 16).view(np.float32)
+        one, per = 0x3F80, 128
+    else:
+        val = lambda bits: bits.astype(np.uint16).view(np.float16).astype(np.float32)
+        one, per = 0x4C00, 1024                          # 2^4: ten binades below it are normal numbers
+    for a in range(one, one + per, 1 if dtype == "bf16" else 3):
+        x = val(np.arange(a - 10 * per, a + 1))
+        got, want = _corrected_codes(np.concatenate([x, -x]), val(np.array([a]))[0])
+        assert np.array_equal(got, want), hex(a)
+    if dtype == "bf16":
+        for binade in (-20, 30, 100, 127):                # far from one: the smallest normal scales, and the largest values
+            for a in (0, 1, 63, 64, 126, 127):
+                bits = ((binade + 127) << 7) + a
+                got, want = _corrected_codes(val(np.arange(bits - 10 * per, bits + 1)), val(np.array([bits]))[0])
+                assert np.array_equal(got, want), hex(bits)
+        tiny = val(np.arange(0, 0x322C))                  # up to 1e-8
+        got, want = _corrected_codes(tiny[tiny <= np.float32(1e-8)], np.float32(0))
+        assert np.array_equal(got, want)
+
