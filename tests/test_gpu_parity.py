@@ -248,21 +248,17 @@ def test_gemm_schedule_grids(cuda_dev, pm, pn):
 def test_gemm_cta_pair_kernel(cuda_dev, M, N, K, dtype, ew):
     """The cta_group::2 kernel forced on for every shape it accepts: odd numbers of 128-row tiles (one CTA of the
     last pair has no rows), ragged N, several tiles per pair, with and without the low-rank term; both epilogue
-    widths (eight warps: long K; sixteen warps: short K) at every shape."""
+    widths (eight warps: long K; sixteen warps: short K) at every shape.  This is the accumulator-dumping instantiation, which
+    stores from registers; the staged store is compared in test_gemm_staged_store_over_many_tiles."""
     _lib.set_option("gemm_pair", 2); _lib.set_option("gemm_epi_warps", ew)
     try:
         run_gemm_case(cuda_dev, M, N, K, lowrank=True, bias=True, dtype=dtype, seed=M + N)
         run_gemm_case(cuda_dev, M, N, K, lowrank=False, bias=True, dtype=dtype, seed=M + N + 1)
-        if ew == 16:                                 # the same tiles stored from registers instead of shared memory + TMA
-            _lib.set_option("gemm_tma_store", 0)
-            run_gemm_case(cuda_dev, M, N, K, lowrank=False, bias=True, dtype=dtype, seed=M + N + 1)
-            _lib.set_option("gemm_tma_store", 1)
         _lib.set_option("gemm_max_ctas", 4)          # two pairs only: long per-pair tile sequences
         run_gemm_case(cuda_dev, M, N, K, lowrank=True, bias=False, dtype=dtype, seed=M + N + 2)
         run_gemm_case(cuda_dev, M, N, K, lowrank=False, bias=False, dtype=dtype, seed=M + N + 3)
     finally:
         _lib.set_option("gemm_pair", 1); _lib.set_option("gemm_max_ctas", 0); _lib.set_option("gemm_epi_warps", 0)
-        _lib.set_option("gemm_tma_store", 1)
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
@@ -526,6 +522,15 @@ def test_shared_input_group(cuda_dev, monkeypatch):
     grp.clear()
 
 
+@pytest.fixture
+def epi_warps(request):
+    """Epilogue warps of the CTA-pair kernel: the epilogue variants take that kernel at every size, sixteen warps at the sizes of
+    these tests and eight in the large launches they stand for."""
+    _lib.set_option("gemm_epi_warps", request.param)
+    yield request.param
+    _lib.set_option("gemm_epi_warps", 0)
+
+
 def _toy_layer(cuda_dev, g, K, N, lowrank=True, bias=True, dtype=torch.bfloat16):
     lin = nn.Linear(K, N, bias=bias).to(dtype)
     with torch.no_grad():
@@ -536,9 +541,10 @@ def _toy_layer(cuda_dev, g, K, N, lowrank=True, bias=True, dtype=torch.bfloat16)
     return int8_exec.Int8Linear(lin, device=cuda_dev, lowrank=lr)
 
 
+@pytest.mark.parametrize("epi_warps", [8, 16], indirect=True)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("N,lowrank", [(768, True), (512, False), (264, True)])
-def test_epilogue_variants(cuda_dev, dtype, N, lowrank):
+def test_epilogue_variants(cuda_dev, dtype, N, lowrank, epi_warps):
     """GELU(tanh) and accumulate-into-output in the GEMM epilogue against the separate torch kernels on the layer's own
     output: the sum bit for bit; the activation within two units in the last place of the output type (hardware tanh).
     N = 264 is a shape the fused variants do not take: same results through the unfused sequence."""
@@ -563,9 +569,10 @@ def test_epilogue_variants(cuda_dev, dtype, N, lowrank):
     assert bool((err <= 4 * ulp * (base + ref_act).float().abs() + 4e-3).all()), err.max().item()
 
 
+@pytest.mark.parametrize("epi_warps", [8, 16], indirect=True)
 @pytest.mark.parametrize("M,K,N,lowrank,copies", [(700, 512, 768, True, 3), (1000, 256, 512, False, 7), (513, 3072, 1024, True, 1),
                                                   (300, 512, 264, True, 2)])
-def test_gemm_stores_to_every_destination(cuda_dev, M, K, N, lowrank, copies):
+def test_gemm_stores_to_every_destination(cuda_dev, M, K, N, lowrank, copies, epi_warps):
     """`forward_into` (pq_int8_gemm_bcast): the epilogue writes each output tile to several buffers -- on several GPUs
     these are the peers' output buffers, here slices of larger local ones.  Every destination must equal the plain
     forward bit for bit and rows outside the slice must stay untouched.  N = 264 is a shape the kernel path does not
@@ -654,9 +661,10 @@ def test_forward_adaln(cuda_dev):
     assert torch.equal(y2, layer.forward_adaln(h[:1], scale[:1], shift[:1])[0])
 
 
+@pytest.mark.parametrize("epi_warps", [8, 16], indirect=True)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("K0,K1,lowrank", [(128, 160, True), (3072, 1024, True), (64, 16, False), (96, 160, True), (15360, 1024, False)])
-def test_forward_on_two_sources(cuda_dev, dtype, K0, K1, lowrank):
+def test_forward_on_two_sources(cuda_dev, dtype, K0, K1, lowrank, epi_warps):
     """`forward_cat(x0, x1)` == the layer on `torch.cat([x0, x1], -1)` (flux/transformer_flux.py:143-145), bit for bit:
     quantisation and down-projection read the two tensors in place.  K0 = 96 (seam off the 64-element grid) and
     K0 + K1 = 16384 (beyond the register-resident rows) take the concatenating route; row-strided views are consumed as
@@ -706,9 +714,10 @@ def test_shared_group_primed_by_adaln(cuda_dev, monkeypatch):
             assert ((a.float() - b.float()).norm() / b.float().norm()).item() < 2e-3
 
 
+@pytest.mark.parametrize("epi_warps", [8, 16], indirect=True)
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("lowrank", [True, False])
-def test_gated_residual_epilogue(cuda_dev, dtype, lowrank):
+def test_gated_residual_epilogue(cuda_dev, dtype, lowrank, epi_warps):
     """`residual + gate.unsqueeze(1) * Linear(x)` (flux/transformer_flux.py:145-149) in the GEMM epilogue: bit-identical to
     the layer followed by torch's multiply and add, two samples with their own gate vectors, fp16 sums clipped as the
     block clips them."""
@@ -1512,3 +1521,63 @@ def test_fuse_rows_keeps_the_background_in_the_graph(cuda_dev):
         dual = fwad.make_dual(bg, torch.ones_like(bg))
         out = fwad.unpack_dual(routing.fuse_rows(dual, y, plan))
         assert torch.equal(out.primal, want) and out.tangent is not None
+
+
+# ------------------------------------------------------------------------------------------------ several streams
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_layers_on_two_streams(cuda_dev, dtype):
+    """Two layers whose forwards overlap on two streams (clusters of several CTAs next to the pair kernel, scratch of both from
+    the allocator) give what they give one after the other, call after call."""
+    g = torch.Generator().manual_seed(12)
+    layers = [_toy_layer(cuda_dev, g, 3072, 1536, lowrank=True, dtype=dtype), _toy_layer(cuda_dev, g, 12288, 768, lowrank=True, dtype=dtype)]
+    xs = [[rand_act(m_rows, m.in_features, dtype, 40 + i).to(cuda_dev) for i, m_rows in enumerate((900, 2100, 70))] for m in layers]
+    want = [[m(x) for x in rows] for m, rows in zip(layers, xs)]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream(cuda_dev) for _ in layers]
+    got = [[], []]
+    for _ in range(8):
+        for i in range(3):
+            for j, (m, st) in enumerate(zip(layers, streams)):
+                with torch.cuda.stream(st):
+                    got[j].append((i, m(xs[j][i])))
+    torch.cuda.synchronize()
+    for j in range(2):
+        assert all(torch.equal(y, want[j][i]) for i, y in got[j])
+    ops.check_device_status(cuda_dev)
+
+
+def test_host_row_pipeline(cuda_dev):
+    """Pinned host rows in and out, two layers' pipelines enqueued before either is awaited: every row as the layer alone
+    computes it, a last chunk that is short, repeated on the same buffers."""
+    from pyraquant_b200.host_pipeline import HostRowPipeline
+    g = torch.Generator().manual_seed(13)
+    M, chunk, dtype = 1000, 384, torch.bfloat16
+    layers = [_toy_layer(cuda_dev, g, 3072, 1024, lowrank=True), _toy_layer(cuda_dev, g, 6144, 512, lowrank=True)]
+    hx = [rand_act(M, m.in_features, dtype, 50 + i).pin_memory() for i, m in enumerate(layers)]
+    hy = [torch.full((M, m.out_features), float("nan"), dtype=dtype).pin_memory() for m in layers]
+    pipes = [HostRowPipeline(m, m.in_features, dtype, cuda_dev, chunk) for m in layers]
+    want = [torch.cat([m(x[a:a + chunk].to(cuda_dev)) for a in range(0, M, chunk)]).cpu() for m, x in zip(layers, hx)]
+    for _ in range(3):
+        for y in hy:
+            y.fill_(float("nan"))
+        for p, x, y in zip(pipes, hx, hy):
+            p.start(x, y)
+        for p in pipes:
+            p.finish()
+        assert all(torch.equal(y, w) for y, w in zip(hy, want))
+    ops.check_device_status(cuda_dev)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_quant_rows_with_infinities(cuda_dev, dtype):
+    """Outside parity, but fixed: a row holding an infinity gets scale NaN and code -1 throughout, a NaN stays in its own row, and
+    the neighbours are what they are without them; the one-launch prologue does the same."""
+    x = rand_act(70, 1024, dtype, 77)
+    clean = x.clone()
+    x[3, 5], x[64, 1000], x[69, 0] = float("inf"), float("-inf"), float("nan")
+    a_t = torch.zeros(32, 1024, dtype=dtype, device=cuda_dev)
+    rows = [r for r in range(70) if r not in (3, 64, 69)]
+    for q, s in (int8_exec.quant_rows(x.to(cuda_dev)), ops.quant_rows_lowrank(x.to(cuda_dev), a_t)[:2]):
+        qo, so = oracle.quant_rows(clean)
+        assert torch.equal(q.cpu()[rows], qo[rows]) and torch.equal(s.cpu()[rows], so[rows])
+        assert bool(s[[3, 64]].isnan().all()) and bool((q[[3, 64]] == -1).all())
