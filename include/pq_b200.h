@@ -248,8 +248,8 @@ int pq_lowrank_down_cat(const void* x0, int64_t K0, int64_t ldx0, const void* x1
                         void* workspace, size_t ws_bytes, void* stream);
 
 /* Quantisation and rank-32 down-projection of the same rows in one launch that reads them once from memory: q, s as
- * pq_quant_rows (bit for bit), t [M, 32] as pq_lowrank_down (same value up to the order of the fp32 summation: the columns
- * are summed in up to eight slices that are then added in order).  The row is x0[m, 0:K0] (K1 == 0), or the concatenation
+ * pq_quant_rows (bit for bit), t [M, 32] as pq_lowrank_down (the same bits: both sum the columns in up to eight slices, a
+ * function of K0 + K1 alone, that are then added in order).  The row is x0[m, 0:K0] (K1 == 0), or the concatenation
  * [x0 | x1] as for the _cat entry points.  R == 32, K0 + K1 <= 16384 (else PQ_ERR_UNSUPPORTED), alignment as there.
  * Replaces the two steps of Int8Linear.forward at deploy/int8_exec.py:388-390. */
 int pq_quant_rows_lowrank(const void* x0, int64_t K0, int64_t ldx0, const void* x1, int64_t K1, int64_t ldx1, int dtype,

@@ -920,11 +920,13 @@ int launch_pair_ew(const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtenso
 }
 
 // Sixteen epilogue warps where the epilogue shows: a short K (the main loop of a tile is over before its epilogue) and
-// launches of few k-blocks per pair, whose last tile's epilogue is a good part of the time.  In long launches, bound by power
-// and not by the epilogue, the eight warps are ahead by 5-8 % (16896 x 3072 -> 12288: 389 / 427 us).  Eight / sixteen, us:
-// without low-rank term 2048 x 8192 -> 4096 56.3 / 50.5, 4608 x 5120 -> 1280 34.5 / 32.4, 16384 x 640 -> 640 24.4 / 13.1;
-// with it 16896 x 1536 -> 6144 171 / 150, 40000 x 1024 -> 2048 114 / 103, 3000 x 3072 -> 1344 21.0 / 19.2,
-// 4608 x 3072 -> 3072 33.6 / 32.8.  Option gemm_epi_warps overrides.
+// launches of few k-blocks per pair, whose last tile's epilogue is a good part of the time.  Long launches are bound by power
+// and not by the epilogue: the two are level (16896 x 3072 -> 12288 402 / 404, 66048 x 3072 -> 3072 393 / 399), with the GELU the
+// eight are ahead (406 / 424, 408 / 444).  Eight / sixteen, bf16, us:
+// staged 16384 x 640 -> 640 26.5 / 14.6, 16384 x 1280 -> 1280 35.4 / 27.1, 16896 x 1536 -> 6144 135 / 115, 2048 x 8192 -> 4096
+// 48.7 / 46.8; two tiers 16896 x 1536 -> 6144 137 / 119, 4608 x 3072 -> 3072 39.4 / 38.8; accumulating 16384 x 1280 -> 1280
+// 71.3 / 48.1, 2048 x 8192 -> 4096 56.8 / 52.3; rank 32 16896 x 1536 -> 6144 156 / 147, 66048 x 1024 -> 2048 198 / 179,
+// 4608 x 3072 -> 3072 35.3 / 34.4, accumulating 56.9 / 43.5.  Option gemm_epi_warps overrides.
 template <typename OutT, bool HAS_LR, bool DBG>
 int launch_pair(const CUtensorMap& tmA, const CUtensorMap& tmW, const CUtensorMap& tmW1, const CUtensorMap& tmT,
                 const CUtensorMap& tmLbT, GemmParams p, int mt_pairs, int ntl, cudaStream_t st) {

@@ -1,7 +1,7 @@
 // Group-32 W8A8 GEMM for sm_100a:
 //   out[m,n] = sum_g s_a[m,g] * s_w[g,n] * (sum_{k in group g} xq[m,k] * w[n,k])  (+ bias[n])
 // A group is 32 consecutive K = exactly one tcgen05.mma kind::i8 instruction, so every instruction produces the exact
-// int32 partial sum of one group in one of four 128-column tensor-memory slots; the epilogue warps drain the slots and
+// int32 partial sum of one group in one of four 128-column (or eight 64-column) tensor-memory slots; the epilogue warps drain the slots and
 // fold them into fp32 running sums in registers: sum = fma(float(partial), s_a * s_w, sum), ascending groups, the
 // arithmetic of the CPU restatement (bit-equal outputs).
 //
@@ -157,7 +157,7 @@ pq_int8_gemm_g32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_co
           tma_load_2d(a_s + L::kABytes, &tmW, &full_bar[stage], kb * BK, n0);
           mbar_arrive_expect_tx(&sfull_bar[stage], L::kScaleBytes);
           tma_load_2d(sc_s, &tmSa, &sfull_bar[stage], kb * kGroupsPerStage, row0);           // [128 rows][4 groups]
-          tma_load_2d(sc_s + L::kSaBytes, &tmSw, &sfull_bar[stage], n0, kb * kGroupsPerStage);  // [4 groups][128 cols]
+          tma_load_2d(sc_s + L::kSaBytes, &tmSw, &sfull_bar[stage], n0, kb * kGroupsPerStage);  // [4 groups][BN cols]
           ++issued;
           if (++stage == kStages) { stage = 0; phase ^= 1u; }
         }

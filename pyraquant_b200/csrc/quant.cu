@@ -6,8 +6,8 @@
 // Arithmetic contract (bit-exact with torch on CPU; deploy/int8_exec.py:508-509 and :83-101):
 //   scale = max(absmax, 1e-8) / 127        IEEE fp32 division
 //   q     = round_half_even(x / scale)     IEEE fp32 division, clamp to [-127, 127]
-// The division per element is a multiplication with the reciprocal and one correction step, exact in every code (see
-// quant_chunk).  Measured against the bracketing form with a divergent exact path that it replaced, back to back over
+// The division per element is a multiplication with the reciprocal and one correction step, exact in every code of a finite row
+// (see quant_chunk; a row with an infinity gets scale NaN and code -1).  Measured against the bracketing form with a divergent exact path that it replaced, back to back over
 // inputs rotating through HBM: 66048 x 3072 bf16 112.5 -> 91.3 us (6.7 TB/s), 16896 x 12288 106.5 -> 92 us, 4608 x 3072
 // 13.3 -> 8.3 us, 65536 x 640 fp16 19.4 -> 16.6 us; group-32 65536 x 2560 fp16 99 -> 82.5 us; behind the adaLN prologue
 // 16896 x 3072 55 -> 45 us.

@@ -27,8 +27,10 @@ __device__ __forceinline__ uint32_t absmax_chunk(uint32_t acc, const uint4& v) {
 // Exact contract: code = round_half_even(fl(x / scale)) with the IEEE quotient.  With inv = fl(1 / scale) correctly
 // rounded, q0 = fl(x * inv), the residual r = fl(x - q0 * scale) and q = fl(q0 + r * inv) give the correctly rounded quotient
 // (Markstein's correction step) short of underflow, where the code is 0 either way; adding 1.5 * 2^23 rounds it to the
-// nearest integer, half to even, and leaves that integer in the low mantissa bits.  The codes were compared with the
-// division's on the host for every pair (absmax, |x| <= absmax) of finite bf16 and of finite fp16 values: no difference.
+// nearest integer, half to even, and leaves that integer in the low mantissa bits.  The tests compare the codes with the
+// division's for every significand of the absmax and every value of the type that can give a code other than 0: no difference.
+// (Not finite: the residual of absmax / 127 is inf - inf, so a row with an infinity gets scale NaN and every code is the low byte
+// of a NaN, -1.)
 // Four packed operations per pair of elements and no branch.  (Bracketing the quotient between two products and redoing
 // a chunk with divisions when they disagree costs the same four operations, but every |x| = absmax / 2 is a rounding tie
 // and took that path: a third of all warp-wide chunks of normally distributed bf16 data.)  No conversion instructions

@@ -20,7 +20,9 @@
 // Measured, bf16, back to back over inputs rotating through HBM, against pq_lowrank_down + pq_quant_rows: 66048 x 15360
 // 742 -> 665 us (4.6 TB/s of the 3 bytes per element), 66048 x 3072 160 -> 136 us, 16896 x 12288 166 -> 141 us,
 // 4608 x 3072 16.0 -> 15.0 us, 512 x 12288 26.5 -> 13.2 us (the down-projection alone has eight 64-row tiles there).  The
-// second sweep bounds it: its sixteen warps wait for L2, then quantise, four rows each per block.  Slower: eight
+// second sweep bounds it: its sixteen warps wait for L2, then quantise, four rows each per block; neither DRAM (48 % at K = 15360)
+// nor L2 (32 %) is near its limit, a scheduler issues 0.6 instructions a cycle from its four warps, and clusters of eight leave
+// 28 of the 148 SMs without a CTA.  Slower: eight
 // quantising warps; the second sweep through a TMA ring of its own (two or three stages are all that fits beside A and
 // cannot cover the L2 latency: 946 us at K = 15360); loading a row's registers ahead of the wait for the maxima (207 us
 // at K = 3072 with clusters); reloading each chunk in place (208 us).

@@ -349,23 +349,28 @@ class Int8Linear(nn.Module):
         return (self.lr_A is not None and self.lr_A.shape[1] == 32 and x2.shape[1] % 32 == 0
                 and self.lr_A.dtype == x2.dtype and self.lr_B.dtype == x2.dtype and self.out_features % 8 == 0)
 
-    def _operand(self, name: str) -> Optional[torch.Tensor]:
-        """``self.<name>`` (a buffer, a Parameter, a plain attribute, a parametrised tensor or None) without the detour through
-        ``nn.Module.__getattr__`` for the usual case of a buffer."""
-        t = self._buffers.get(name)
-        return t if t is not None else getattr(self, name)
-
     def _lean_forward(self, x2: torch.Tensor):
         """Eager fast path for the common case (aligned rows, no branch or a rank-32 one): one C-ABI call with the per-layer
         constants in a descriptor, skipping the generic wrappers' checks; for rows whose down-projection does not share the
         quantisation's launch the three calls are made from here.  Returns None when the input does not qualify."""
         M, K = x2.shape
         dt = x2.dtype
-        w = self._operand("weight_int8")
+        # the layer's tensors as `self.<name>` gives them -- buffers, Parameters, plain attributes, parametrised tensors -- without
+        # the detour through nn.Module.__getattr__ (0.3 us each) for the usual case of a buffer
+        bufs = self._buffers
+        w = bufs.get("weight_int8")
+        if w is None:
+            w = self.weight_int8
         if (M == 0 or not x2.is_cuda or x2.stride(1) != 1 or x2.stride(0) % 8 or x2.data_ptr() % 16 or K % 16
                 or x2.device != w.device or dt not in ops._DT or torch.compiler.is_compiling()):
             return None
-        lr_a, bias = self._operand("lr_A"), self._operand("bias")
+        lr_a, bias, sc = bufs.get("lr_A"), bufs.get("bias"), bufs.get("w_scale")
+        if lr_a is None:
+            lr_a = self.lr_A
+        if bias is None:
+            bias = self.bias
+        if sc is None:
+            sc = self.w_scale
         rank = 0
         low = None
         one_launch = True
@@ -382,7 +387,6 @@ class Int8Linear(nn.Module):
             low = (lr_b.data_ptr(), lbt.data_ptr(), at.data_ptr() if one_launch else None)
         # every buffer whose address is cached takes part in the key: .to(dtype) / .half() / load_state_dict(assign=True)
         # replace the float buffers while the int8 weight stays where it is
-        sc = self._operand("w_scale")
         key = (w.data_ptr(), dt, sc.data_ptr(), bias.data_ptr() if bias is not None else 0, low)
         c = self.__dict__.get("_lean_cache")
         if c is None or c[0] != key:
