@@ -251,6 +251,7 @@ int pq_lowrank_down_cat(const void* x0, int64_t K0, int64_t ldx0, const void* x1
  * pq_quant_rows (bit for bit), t [M, 32] as pq_lowrank_down (the same bits: both sum the columns in up to eight slices, a
  * function of K0 + K1 alone, that are then added in order).  The row is x0[m, 0:K0] (K1 == 0), or the concatenation
  * [x0 | x1] as for the _cat entry points.  R == 32, K0 + K1 <= 16384 (else PQ_ERR_UNSUPPORTED), alignment as there.
+ * (Few short rows under stream capture: the two kernels of the separate entry points, which take less time on the device.)
  * Replaces the two steps of Int8Linear.forward at deploy/int8_exec.py:388-390. */
 int pq_quant_rows_lowrank(const void* x0, int64_t K0, int64_t ldx0, const void* x1, int64_t K1, int64_t ldx1, int dtype,
                           int64_t M, const void* a_t, int64_t lda, int R, int8_t* q, float* s, void* t, int64_t ldt,

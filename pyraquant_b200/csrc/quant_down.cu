@@ -476,6 +476,19 @@ int lowrank_slice_blocks(int64_t K) {
 }  // namespace pq
 
 namespace {
+// Short rows in a launch of few: the two kernels one after the other run for less time than the one (whose set-up, exchange and
+// second sweep are a chain that small blocks do not hide), but the extra launch costs the host more than that (4 us a call of the
+// eager forward).  So they are taken where the launches are recorded and the host's time is not in the way: under stream capture.
+// Device time of the whole forward, one launch / two, us: 154 x 640 -> 1280 14.7 / 12.3, 1024 x 1536 -> 1536 20.3 / 16.1, 8256 x 512
+// -> 512 17.6 / 16.9; host time of the eager call 22.8 / 26.6.  From the row counts below on the one is ahead (16384 x 1024 -> 1024
+// 47.4 / 47.3, 65536 x 640 -> 1280 132.7 / 133.0).  Codes, scales and t are the same bits either way.
+bool two_launches(int64_t M, int64_t K, cudaStream_t st) {
+  if (K > 1536 || M >= (K < 768 ? 65536 : 16384)) return false;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &capture) != cudaSuccess) { cudaGetLastError(); return false; }
+  return capture == cudaStreamCaptureStatusActive;
+}
+
 // q == nullptr: t only
 int quant_down_impl(const void* x0, int64_t K0, int64_t ldx0, const void* x1, int64_t K1, int64_t ldx1, int dtype, int64_t M,
                     const void* a_t, int64_t lda, int R, int8_t* q, float* s, void* t, int64_t ldt, void* workspace,
@@ -493,6 +506,14 @@ int quant_down_impl(const void* x0, int64_t K0, int64_t ldx0, const void* x1, in
   if (K1 > 0 && (K1 % 8 != 0 || ldx1 % 8 != 0 || !aligned_to(x1, 16))) return PQ_ERR_ALIGN;
   if (K1 > 0 && K0 % QKE != 0) return PQ_ERR_UNSUPPORTED;       // the seam has to fall between two boxes
   if (workspace != nullptr && ws_bytes < PQ_GEMM_WORKSPACE_BYTES) return PQ_ERR_WORKSPACE;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (q != nullptr && two_launches(M, K, st)) {
+    const int rc = K1 > 0 ? pq_lowrank_down_cat(x0, K0, ldx0, x1, K1, ldx1, dtype, a_t, lda, R, t, ldt, M, workspace, ws_bytes, stream)
+                          : pq_lowrank_down(x0, dtype, ldx0, a_t, lda, R, t, ldt, M, K, workspace, ws_bytes, stream);
+    if (rc != PQ_OK) return rc;
+    return K1 > 0 ? pq_quant_rows_cat(x0, K0, ldx0, x1, K1, ldx1, dtype, M, q, s, stream)
+                  : pq_quant_rows(x0, dtype, M, K, ldx0, q, s, stream);
+  }
   const bool bf16 = dtype == PQ_DTYPE_BF16;
   CUtensorMap tmX, tmX1, tmA;
   int rc = make_map16(&tmX, x0, M, K0, ldx0, QM, bf16);
@@ -516,7 +537,6 @@ int quant_down_impl(const void* x0, int64_t K0, int64_t ldx0, const void* x1, in
   const int cl = cluster_size(K);
   p.kb_slice = lowrank_slice_blocks(K);
   p.stages = 0;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (K1 > 0) {
     if (bf16) return launch_qd_cl<__nv_bfloat16, true>(cl, tmX, tmX1, tmA, p, st);
     return launch_qd_cl<__half, true>(cl, tmX, tmX1, tmA, p, st);

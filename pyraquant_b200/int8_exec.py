@@ -381,7 +381,7 @@ class Int8Linear(nn.Module):
             one_launch = ops.quant_lowrank_ok(x2)              # else: rows too short or too long for the shared launch
             lr_b, lbt, at = self.lr_B, self._lr_Bt(), self._lr_At() if one_launch else None
             # the library sees bare pointers: factors that do not fit the layer must not get there
-            assert at is None or (at.shape == (32, K) and at.device == x2.device), (tuple(at.shape), at.device)
+            assert at is None or (at.numel() == 32 * K and at.get_device() == x2.get_device()), (tuple(at.shape), at.device)
             if lr_b.stride(1) != 1:
                 return None
             low = (lr_b.data_ptr(), lbt.data_ptr(), at.data_ptr() if one_launch else None)

@@ -1523,6 +1523,37 @@ def test_fuse_rows_keeps_the_background_in_the_graph(cuda_dev):
         assert torch.equal(out.primal, want) and out.tangent is not None
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,K1", [(70, 512, 0), (1025, 736, 0), (300, 1536, 0), (300, 1568, 0), (130, 640, 384)])
+def test_quant_rows_lowrank_under_capture(cuda_dev, M, K, K1, dtype):
+    """Codes, scales and t recorded in a graph (few short rows: as two kernels) are those of the eager call (one kernel), and a
+    replay reads the rows anew; one and two sources, a row length on either side of the line; the layer's forward as well."""
+    g = torch.Generator().manual_seed(M + K)
+    Kt = K + K1
+    x = rand_act(M, Kt, dtype, M).to(cuda_dev)
+    other = rand_act(M, Kt, dtype, M + 1).to(cuda_dev)
+    m = _toy_layer(cuda_dev, g, Kt, 264, lowrank=True, dtype=dtype)
+    a_t = m._lr_At()
+    parts = (lambda v: (v[:, :K].contiguous(), v[:, K:].contiguous())) if K1 else (lambda v: (v, None))
+    want = []
+    for v in (x, other):
+        x0, x1 = parts(v)
+        want.append((*ops.quant_rows_lowrank(x0, a_t, x1), m(v)))
+    x0, x1 = parts(x)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = (*ops.quant_rows_lowrank(x0, a_t, x1), m(x))
+    for v, w in zip((x.clone(), other), want):
+        x.copy_(v)
+        if K1:
+            x0.copy_(v[:, :K]); x1.copy_(v[:, K:])
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(a, b) for a, b in zip(got, w))
+    ops.check_device_status(cuda_dev)
+
+
 # ------------------------------------------------------------------------------------------------ several streams
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_layers_on_two_streams(cuda_dev, dtype):
